@@ -227,6 +227,11 @@ def _prepare_step(case, g):
     return s
 
 
+def _linear_weights(case, g):
+    out, inp = case["out"], case["in"]
+    return [(_codes(g, out, inp), _scales(g, out // 128, 0.1), _zeros(g, out // 128, case["integral"])) for _ in range(case["count"])]
+
+
 def prepare(case, seed):
     family = case["family"]
     g = _generator(seed)
@@ -243,8 +248,7 @@ def prepare(case, seed):
         return {"family": family, "ops": ops, "heads": heads, "rows": rows, "pos0": pos0, "max_pos": max_pos,
                 "qkv": _normal(g, rows, 3 * heads * 128), "k": _normal(g, heads, max_pos, 128), "v": _normal(g, heads, max_pos, 128)}
     out, inp, count = case["out"], case["in"], case["count"]
-    weights = [ops.W4Linear(_codes(g, out, inp), _scales(g, out // 128, 0.1), _zeros(g, out // 128, case["integral"]), out, inp,
-                            zp_integral=case["integral"]) for _ in range(count)]
+    weights = [ops.W4Linear(*w, out, inp, zp_integral=case["integral"]) for w in _linear_weights(case, g)]
     s = {"family": family, "ops": ops, "ws": ops.Workspace(), "weights": weights}
     if family == "rows":
         s["x"] = _normal(g, case["rows"], inp)
@@ -343,3 +347,52 @@ def tolerance(case):
     if case["family"] in ("generate", "step"):
         return {"rel": 1e-2, "max": 0.1, "differ": 0.0}
     return {"rel": 1e-3, "max": 4e-3}
+
+
+# ---- the same results in 64 bits, in plain torch ---------------------------------------------------------------------------------
+
+def _exact_product(packed, scale, zp, out, inp, x):
+    """x (rows of float64) times the dequantised matrix.  The weights themselves are fp16 by definition: fp16(fp16(q - zp) * scale)."""
+    y = torch.empty(x.shape[0], out, dtype=torch.float64, device="cuda")
+    j = torch.arange(inp, device="cuda")
+    for b0 in range(0, out // 128, 32):   # 4096 outputs at a time
+        b1 = min(b0 + 32, out // 128)
+        block = packed.view(inp, out // 2)[:, 64 * b0:64 * b1]
+        q = torch.stack((block & 15, block >> 4), 2).view(inp, -1, 128).half()
+        group = ((torch.arange(b0, b1, device="cuda")[None, :] + j[:, None] * (out // 128)) % (inp // 128)) % scale.numel()
+        w = (q - zp[group][:, :, None]) * scale[group][:, :, None]
+        y[:, 128 * b0:128 * b1] = x @ w.view(inp, -1).double()
+    return y
+
+
+def exact(case, seed):
+    """Linears, row blocks and attention.  A token pass rounds to fp16 between its operators by definition, and which logit
+    wins decides what comes next: it has no 64-bit result that an implementation could come nearer to."""
+    family = case["family"]
+    if family in ("generate", "step"):
+        return None
+    g = _generator(seed)
+    if family == "attention":
+        heads, rows, pos0 = case["heads"], case["rows"], case["pos0"]
+        max_pos = -(-(pos0 + rows) // 128) * 128
+        qkv, k, v = _normal(g, rows, 3 * heads * 128), _normal(g, heads, max_pos, 128), _normal(g, heads, max_pos, 128)
+        hidden = torch.arange(pos0 + rows, device="cuda")[None, :] > pos0 + torch.arange(rows, device="cuda")[:, None]
+        y = torch.empty(rows, heads * 128, dtype=torch.float64, device="cuda")
+        for h in range(heads):
+            s = qkv[:, 128 * h:128 * h + 128].double() @ k[h, :pos0 + rows].double().T / math.sqrt(128.0)
+            y[:, 128 * h:128 * h + 128] = torch.softmax(s.masked_fill(hidden, -math.inf), 1) @ v[h, :pos0 + rows].double()
+        return y
+    out, inp = case["out"], case["in"]
+    weights = _linear_weights(case, g)
+    if family == "rows":
+        x = _normal(g, case["rows"], inp).double()
+        return [_exact_product(*w, out, inp, x) for w in weights]
+    x = _normal(g, inp)
+    if case["epilogue"] != "store":   # the normalised vector is fp16 by definition, as its factor is: fp16(fp16(x * r) * gamma)
+        gamma = _normal(g, inp, mean=1.0, std=0.02)
+        r = (1.0 / torch.sqrt(x.double().square().mean() + 1e-6)).half()
+        x = x * r * gamma
+    ys = [_exact_product(*w, out, inp, x.double()[None, :])[0] for w in weights]
+    if case["epilogue"] == "gelu":   # of the product as fp16
+        ys = [0.5 * y * (1.0 + torch.erf(y * math.sqrt(0.5))) for y in (y.half().double() for y in ys)]
+    return ys
