@@ -20,7 +20,7 @@
 #include <cstdlib>
 #include <mutex>
 
-#include "common.cuh"
+#include "tc05.cuh"
 
 namespace qw3 {
 
@@ -60,51 +60,6 @@ struct GemmParams {
     int a_lbo, a_sbo, a_kstep;   // operand A descriptor: byte offsets between 64-output blocks, between 8-deep K blocks, per K=16 step
 };
 
-__device__ __forceinline__ uint32_t elect_one() {
-    uint32_t pred;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "elect.sync _|p, 0xffffffff;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(pred));
-    return pred;
-}
-
-// Shared-memory matrix descriptor (tcgen05): start >> 4 in bits 0-13, leading byte offset >> 4 in
-// bits 16-29, stride byte offset >> 4 in bits 32-45, version 1 in bits 46-47, swizzle mode in bits 61-63
-// (2 = 128-byte swizzle).
-__device__ __forceinline__ uint64_t make_smem_desc(uint32_t smem_addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
-    uint64_t d = 0;
-    d |= (uint64_t)((smem_addr & 0x3FFFFu) >> 4);
-    d |= (uint64_t)((lbo_bytes >> 4) & 0x3FFFu) << 16;
-    d |= (uint64_t)((sbo_bytes >> 4) & 0x3FFFu) << 32;
-    d |= (uint64_t)1 << 46;
-    d |= (uint64_t)2 << 61;
-    return d;
-}
-
-__device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr) : "memory");
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
 // One output element: fp32 sum -> fp16, then the epilogue in fp16 as the decode path does it.
 __device__ __forceinline__ __half gemm_epilogue(float v, int epilogue, __half old) {
     const __half h = __float2half_rn(v);
@@ -129,7 +84,7 @@ gemm_w4a16_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const GemmParam
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 6 * GM_MAX_STAGES + 1);
     int* s_dead = reinterpret_cast<int*>(tmem_slot + 1);   // bars: (6 * 24 + 2) * 8 bytes < 1280
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
     const int tile_m = blockIdx.x, tile_n = blockIdx.y;
     // split-K: grid.z CTAs share the K blocks of a tile; each handles [kb_lo, kb_lo + n_kb)
     const int n_kb_all = p.K / GM_BK;
@@ -161,7 +116,7 @@ gemm_w4a16_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const GemmParam
         // ---------------- TMA producer of the activations ------------------------------------------
         // (the packed nibbles do not go through TMA: a 128-output tile is 64 bytes wide, and a box of 64 such rows
         // cost the copy engine more per K block than everything else in the CTA)
-        if (lane == 0) {
+        if (elect_one()) {
             tma_prefetch_desc(&tmap_x);
             bool ok = true;
             for (int kb = 0; kb < n_kb && ok; ++kb) {
@@ -182,7 +137,7 @@ gemm_w4a16_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const GemmParam
         // K block costs a CTA when the row tile is small, so TWO warps issue: warp 1 takes the even K blocks, the
         // last warp the odd ones, each into its own accumulators (summed by the epilogue).  One lane per warp runs
         // the loop; ring indices and phases are running counters, descriptors a constant plus additions.
-        if (lane == 0) {
+        if (elect_one()) {
             const int who = warp == 1 ? 0 : 1;
             // instruction descriptor: D = f32, A = B = f16, A MN-major (bit 15), B K-major, N >> 3, M >> 4
             const uint32_t idesc = (1u << 4) | (1u << 15) | ((uint32_t)(p.n_tile >> 3) << 17) | ((uint32_t)(GM_TILE_M >> 4) << 24);
@@ -368,8 +323,7 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-static int encode_2d(CUtensorMap* map, CUtensorMapDataType dt, const void* base, uint64_t inner, uint64_t outer,
-                     uint64_t pitch_bytes, uint32_t box_inner, uint32_t box_outer, CUtensorMapSwizzle swz) {
+int encode_f16_map(CUtensorMap* map, const void* base, int rank, const uint64_t* dims, const uint64_t* strides, const uint32_t* box) {
     static EncodeTiledFn fn = nullptr;
     static std::once_flag once;
     std::call_once(once, [] {
@@ -383,17 +337,26 @@ static int encode_2d(CUtensorMap* map, CUtensorMapDataType dt, const void* base,
         set_last_error("cuTensorMapEncodeTiled is not available (no CUDA driver?)");
         return QW3_ERR_CUDA;
     }
-    cuuint64_t dims[2] = {inner, outer};
-    cuuint64_t strides[1] = {pitch_bytes};
-    cuuint32_t box[2] = {box_inner, box_outer};
-    cuuint32_t estr[2] = {1, 1};
-    CUresult r = fn(map, dt, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swz,
-                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    cuuint64_t d[3], s[2] = {0, 0};
+    cuuint32_t b[3], estr[3] = {1, 1, 1};
+    for (int i = 0; i < rank; ++i) {
+        d[i] = dims[i];
+        b[i] = box[i];
+        if (i + 1 < rank) s[i] = strides[i];
+    }
+    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, (cuuint32_t)rank, const_cast<void*>(base), d, s, b, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) {
         set_last_error("cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
         return QW3_ERR_CUDA;
     }
     return QW3_OK;
+}
+// Activation rows [rows][K] in boxes of 64 inputs x box_rows.
+static int encode_rows(CUtensorMap* map, const void* x, int64_t rows, int64_t K, int box_rows) {
+    const uint64_t dims[2] = {(uint64_t)K, (uint64_t)rows}, strides[1] = {(uint64_t)K * 2};
+    const uint32_t box[2] = {GM_BK, (uint32_t)box_rows};
+    return encode_f16_map(map, x, 2, dims, strides, box);
 }
 
 }  // namespace qw3
@@ -431,8 +394,7 @@ int qw3::gemm_launch(qw3_w4_t w, const void* d_x, int64_t rows, void* d_y, qw3_w
     p.a_lbo = 8192; p.a_sbo = 1024; p.a_kstep = 2048;
     CUtensorMap tmap_x;
     int rc;
-    rc = encode_2d(&tmap_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, d_x, (uint64_t)d->K, (uint64_t)rows, (uint64_t)d->K * 2, GM_BK,
-                   (uint32_t)p.n_tile, CU_TENSOR_MAP_SWIZZLE_128B);
+    rc = encode_rows(&tmap_x, d_x, rows, d->K, p.n_tile);
     if (rc != QW3_OK) return rc;
     // shared memory per stage: 16 KB of operand A + n_tile x 128 bytes of activations; 6 stages (4 with 256-row tiles)
     const int stages = p.n_tile <= 128 ? 6 : 4;

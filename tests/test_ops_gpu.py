@@ -68,6 +68,28 @@ def test_attention_prefill_block(ops, orc, cuda, heads, max_pos, pos0, rows):
         assert (_ulp_diff(got[r], want) > 1).mean() < 0.01, r
 
 
+@pytest.mark.parametrize("heads,max_pos,pos0,rows", [(1, 128, 0, 65), (2, 512, 0, 128), (2, 700, 63, 193), (1, 1400, 1000, 257),
+                                                     (3, 640, 64, 512), (2, 577, 320, 256)])
+def test_attention_prefill_pairs_of_row_tiles(ops, orc, cuda, heads, max_pos, pos0, rows):
+    """Two tiles of 128 rows against 64-key tiles: ends inside a row tile and a key tile, scores whose maximum grows along the cache
+    by far more than the eight powers of two after which the sums are rescaled, and NaN behind the last row of the
+    block, which nothing may read."""
+    H = heads * 128
+    qkv = orc.gen_normal_f16(31, orc.ACT, rows * 3 * H).reshape(rows, 3 * H)
+    kc = orc.gen_normal_f16(31, orc.KV_K, heads * max_pos * 128).reshape(heads, max_pos, 128).copy()
+    vc = orc.gen_normal_f16(31, orc.KV_V, heads * max_pos * 128).reshape(heads, max_pos, 128).copy()
+    kc *= np.linspace(0.2, 6.0, max_pos, dtype=np.float32).astype(np.float16)[None, :, None]
+    kc[:, pos0 + rows:] = np.nan
+    vc[:, pos0 + rows:] = np.nan
+    got = ops.attn_prefill(_to_dev(qkv, cuda), _to_dev(kc.ravel(), cuda), _to_dev(vc.ravel(), cuda), heads, max_pos, pos0, rows).cpu().numpy()
+    for r in sorted(set([0, 1, 31, 63, 64, 127, 128, rows // 2, rows - 2, rows - 1]) & set(range(rows))):
+        want = orc.attention(np.ascontiguousarray(qkv[r, :H]), kc.ravel(), vc.ravel(), heads, 128, max_pos, pos0 + r + 1)
+        err = np.abs(got[r].astype(np.float32) - want.astype(np.float32))
+        assert (err <= 2e-2 * np.abs(want.astype(np.float32)) + 2e-3).all(), r
+        assert (_ulp_diff(got[r], want) > 1).mean() < 0.01, r
+
+
+
 def test_embed_gather_bit_exact(ops, orc, cuda):
     H, V = 512, 4096 + 256
     p, s, z = orc.gen_linear(24, H, V, kind=orc.EMB)
