@@ -36,6 +36,7 @@ void set_last_error(const char* fmt, ...);
 constexpr int WS_TILE = 1024;          // outputs per GEMV tile
 constexpr int WS_MAX_CTAS = 256;       // upper bound on the GEMV grid
 constexpr int WS_MAX_TILES = 2048;     // upper bound on out_dim / WS_TILE
+constexpr size_t WS_PARTIALS = (size_t)(WS_MAX_CTAS + WS_MAX_TILES) * WS_TILE;   // floats
 constexpr int WS_ATT_MAX_HEADS = 128;
 constexpr int WS_ATT_MAX_SPLITS = 32;
 constexpr int WS_ATT_STRIDE = 132;     // head_dim (128) outputs + running max + running sum + pad

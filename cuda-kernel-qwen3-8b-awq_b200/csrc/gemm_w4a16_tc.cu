@@ -318,6 +318,434 @@ __global__ void gemm_splitk_reduce_kernel(const float* __restrict__ part, int sp
         __halves2half2(gemm_epilogue(acc.x, epilogue, __low2half(old)), gemm_epilogue(acc.y, epilogue, __high2half(old)));
 }
 
+// ---- CTA pairs ------------------------------------------------------------------------------------------------------------------
+// More than 128 rows, or more output tiles than pairs (pair_wanted).  2048 rows of 12288 x 4096: 246 us before, 189 now (0.65 of the
+// measured bf16 rate); 64 rows of 151936 x 4096: 264 before, 205 now.  Bound: a K block takes 0.35 us from the unpack warps to the
+// freed stage whatever the row count (0.25 us with the unpacking left out), above the 0.28 us its MMAs take at 256 rows.
+// Two SMs of a cluster work on one tile of 256 outputs x n_tile rows (tcgen05 cta_group::2): each CTA unpacks operand A for its
+// own 128 outputs and holds half of the activation rows, so that a K block moves half the operand-B bytes through an SM's
+// shared memory (A 16 KB written + 16 KB read, B 16 KB + 16 KB, in the 512 cycles the MMAs take at 256 rows) and half through L2.
+//   warp 0      TMA producer of this CTA's half of the activation rows
+//   warp 1      MMA issuer (leader CTA of the pair only), even / odd K blocks into two accumulators
+//   warps 2..17 unpack (four groups of four warps take the K blocks in turn), epilogue
+//   warp 18     loader: the packed bytes of this CTA's outputs into a ring of twelve K blocks (cp.async, 64 bytes of a row; a tensor
+//               copy of such a narrow box costs more than all else in the CTA).  The unpack warps must not have loads
+//               from global memory in flight: the fence that hands operand A to the tensor cores waits for them.
+// Operand A is K-major: a thread takes 8 outputs x 8 inputs (one 32-bit word of eight rows); a byte permute joins
+// the same byte of two neighbouring rows, and the masks that pick the nibbles then give half2 pairs along K with no
+// more instructions than pairs along the outputs cost.  Row m of A holds output 8 (m & 15) + (m >> 4) of its block, which
+// makes the 16-byte stores of a warp free of bank conflicts; the epilogue undoes it through a staging tile and stores
+// 16 bytes a thread.  The pairs are persistent and take the work items (tile x K split) round robin.
+constexpr int GP_STAGES = 5;
+constexpr int GP_PK_STAGES = 12, GP_PK_BYTES = GM_BK * 64;           // ring of packed K blocks: 48 KB on the way to an SM
+constexpr int GP_MAX_N = 256;
+constexpr int GP_X_BYTES = GP_MAX_N / 2 * 128;                       // this CTA's half of the activation rows, 64 deep
+constexpr int GP_WARPS = 16, GP_GROUPS = GP_WARPS / 4;
+constexpr int GP_LOADER = 2 + GP_WARPS;                              // warp index of the loader of packed bytes
+constexpr int GP_THREADS = 32 * (GP_LOADER + 1);
+constexpr int GP_STG_LD = 136;                                       // halves per staged row: 272 B, 16-byte pieces of a row aligned
+constexpr int GP_STG_BYTES = 16 * GP_STG_LD * 2;                     // 16 rows x 128 outputs per group
+constexpr int GP_TAB = 256;                                          // groups of a column: in_dim / 128 <= 256
+constexpr size_t GP_SMEM = (size_t)GP_STAGES * (GM_A_BYTES + GP_X_BYTES) + GP_PK_STAGES * GP_PK_BYTES + GP_GROUPS * GP_STG_BYTES + GP_TAB * 4 + 512;
+
+struct PairParams {
+    const uint8_t* packed;
+    const __half* scale;
+    const __half* zp;
+    int n_alloc, M, K, Mb, Kb;
+    int rows, n_tile, n_tiles_n, n_tiles_m;
+    int full;          // tiles whose K is not split
+    int splits;        // parts of the K of each of the tiles after those
+    int items;         // full + splits * (the other tiles)
+    int epilogue;
+    __half* y;         // [rows][M]
+    float* part;       // partial products of the split tiles: [tile][split][n_tile][256] in the order of A's rows
+    int* err;
+};
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Arrive on the barrier at the same shared-memory offset in the pair's leader (rank 0; the leader itself included).  What is handed
+// over lies in this CTA's own shared or tensor memory and has been fenced for the tensor cores, which alone read it: a
+// release at cluster scope would add a memory barrier that is longer than the unpacking.
+__device__ __forceinline__ void mbar_arrive_leader(uint32_t bar) {
+    asm volatile(
+        "{\n\t.reg .b32 a;\n\t"
+        "mapa.shared::cluster.u32 a, %0, 0;\n\t"
+        "mbarrier.arrive.shared::cluster.b64 _, [a];\n\t}"
+        ::"r"(bar) : "memory");
+}
+// Box of the tensor map into this CTA's shared memory, completing on the leader's barrier (bit 24 of a shared::cluster address
+// is the CTA's place in the pair).
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+        ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar & 0xFEFFFFFFu) : "memory");
+}
+__device__ __forceinline__ void umma_f16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {   // arrives at the same offset in both CTAs
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                 ::"r"(bar), "h"((unsigned short)3) : "memory");
+}
+__device__ __forceinline__ uint32_t h2_add(uint32_t a, uint32_t b) {
+    uint32_t r;
+    asm("add.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
+    uint32_t r;
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(sel));
+    return r;
+}
+
+// One work item: tile and K range.  Neighbouring items share the 256 outputs and differ in the rows.
+struct PairItem { int tile_m, tile_n, kb_lo, n_kb, slot; };   // slot: place of the partial products, negative: none
+__device__ __forceinline__ PairItem pair_item(const PairParams& p, int item) {
+    PairItem w;
+    const int n_kb = p.K / GM_BK;
+    int tile = item;
+    w.kb_lo = 0;
+    w.n_kb = n_kb;
+    w.slot = item - p.full;
+    if (w.slot >= 0) {
+        const int z = w.slot % p.splits;
+        tile = p.full + w.slot / p.splits;
+        w.kb_lo = z * n_kb / p.splits;
+        w.n_kb = (z + 1) * n_kb / p.splits - w.kb_lo;
+    }
+    w.tile_n = tile % p.n_tiles_n;
+    w.tile_m = tile / p.n_tiles_n;
+    return w;
+}
+// Barrier of the four warps of a group that tells all of them whether one has given up.
+__device__ __forceinline__ bool group_any(int id, bool v) {
+    uint32_t r;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.u32 p, %2, 0;\n\t"
+        "barrier.cta.red.or.aligned.pred q, %1, 128, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(r) : "r"(id), "r"((uint32_t)v) : "memory");
+    return r != 0;
+}
+
+template <bool EXACT, bool UNIFORM>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
+gemm_w4a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const PairParams p) {
+    extern __shared__ __align__(1024) uint8_t smem[];
+    uint8_t* a_st = smem;
+    uint8_t* x_st = a_st + GP_STAGES * GM_A_BYTES;
+    uint8_t* pk_st = x_st + GP_STAGES * GP_X_BYTES;
+    uint8_t* stg = pk_st + GP_PK_STAGES * GP_PK_BYTES;
+    uint32_t* tab = reinterpret_cast<uint32_t*>(stg + GP_GROUPS * GP_STG_BYTES);   // (zero point, scale) of a group
+    uint64_t* bars = reinterpret_cast<uint64_t*>(tab + GP_TAB);
+    const uint32_t a_full = smem_u32(bars), x_full = smem_u32(bars + GP_STAGES), st_empty = smem_u32(bars + 2 * GP_STAGES);
+    const uint32_t acc_full = smem_u32(bars + 3 * GP_STAGES), acc_empty = smem_u32(bars + 3 * GP_STAGES + 1);
+    const uint32_t pk_full = smem_u32(bars + 3 * GP_STAGES + 2), pk_empty = pk_full + 8 * GP_PK_STAGES;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 3 * GP_STAGES + 2 + 2 * GP_PK_STAGES);
+    volatile int* s_dead = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+    const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
+    const int rank = (int)cluster_rank();
+    const int first = blockIdx.x >> 1, step = gridDim.x >> 1, items = p.items;
+
+    if (tid == 0) {
+        for (int s = 0; s < GP_STAGES; ++s) {
+            mbar_init(a_full + 8 * s, 8);       // four unpack warps of each CTA (used in the leader)
+            mbar_init(x_full + 8 * s, 1);       // the leader's expect; bytes of both CTAs' copies
+            mbar_init(st_empty + 8 * s, 1);     // commit of the MMAs that read the stage
+        }
+        for (int s = 0; s < GP_PK_STAGES; ++s) {
+            mbar_init(pk_full + 8 * s, 32);     // the loader's lanes, each when its copies have landed
+            mbar_init(pk_empty + 8 * s, 4);     // the warps of the group that took the block
+        }
+        mbar_init(acc_full, 1);                 // commit of an item's last MMAs
+        mbar_init(acc_empty, 2 * GP_WARPS);     // every epilogue warp of the pair has read its share
+        *s_dead = 0;
+        mbar_fence_init();
+    }
+    for (int g = tid; g < p.Kb; g += GP_THREADS) tab[g] = pack_h2(p.zp[g % p.n_alloc], p.scale[g % p.n_alloc]);
+    if (warp == 1) {   // all 512 columns: two accumulators of up to 256
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();   // the peer's barriers are initialised before anything arrives on them
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+
+    if (warp == 0) {
+        if (elect_one()) {
+            tma_prefetch_desc(&tmap_x);
+            const int half_n = p.n_tile / 2;
+            int s = 0;
+            uint32_t phase = 0;
+            bool ok = true, wrapped = false;
+            for (int item = first; item < items && ok; item += step) {
+                const PairItem w = pair_item(p, item);
+                for (int kb = 0; kb < w.n_kb; ++kb) {
+                    if (wrapped && !(ok = mbar_wait(st_empty + 8 * s, phase ^ 1u))) break;
+                    if (*s_dead != 0) { ok = false; break; }
+                    if (rank == 0) mbar_expect_tx(x_full + 8 * s, (uint32_t)p.n_tile * 128u);
+                    tma_load_2d_pair(smem_u32(x_st + s * GP_X_BYTES), &tmap_x, (w.kb_lo + kb) * GM_BK,
+                                     w.tile_n * p.n_tile + rank * half_n, x_full + 8 * s);
+                    if (++s == GP_STAGES) { s = 0; phase ^= 1u; wrapped = true; }
+                }
+            }
+            // drain: the release arrivals of the last laps land before this CTA may leave
+            for (int t = 0; t < GP_STAGES && ok; ++t)
+                if (t < s || wrapped) ok = mbar_wait(st_empty + 8 * t, t < s ? phase : phase ^ 1u);
+            if (!ok) {
+                atomicCAS(p.err, 0, 0x30011);
+                *s_dead = 1;
+            }
+        }
+        __syncwarp();
+    } else if (warp == 1) {
+        if (rank == 0 && elect_one()) {
+            // D = f32, A = B = f16, both K-major, N >> 3, M >> 4
+            const uint32_t idesc = (1u << 4) | ((uint32_t)(p.n_tile >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
+            const uint64_t adesc0 = make_smem_desc(smem_u32(a_st), 16, 1024), bdesc0 = make_smem_desc(smem_u32(x_st), 16, 1024);
+            int s = 0, n = 0;
+            uint32_t phase = 0;
+            bool ok = true;
+            for (int item = first; item < items && ok; item += step, ++n) {
+                const PairItem w = pair_item(p, item);
+                if (n > 0 && !(ok = mbar_wait(acc_empty, (uint32_t)(n - 1) & 1u))) break;
+                tc_fence_after();
+                for (int kb = 0; kb < w.n_kb; ++kb) {
+                    if (*s_dead != 0 || !mbar_wait(x_full + 8 * s, phase) || !mbar_wait(a_full + 8 * s, phase)) {
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    const uint64_t adesc = adesc0 + (uint64_t)(uint32_t)(s * (GM_A_BYTES >> 4));
+                    const uint64_t bdesc = bdesc0 + (uint64_t)(uint32_t)(s * (GP_X_BYTES >> 4));
+                    const uint32_t d = tmem_base + (uint32_t)((kb & 1) * GP_MAX_N);
+#pragma unroll
+                    for (int ks = 0; ks < GM_BK / 16; ++ks)
+                        umma_f16_pair(d, adesc + (uint64_t)(2 * ks), bdesc + (uint64_t)(2 * ks), idesc, (kb >= 2 || ks > 0) ? 1u : 0u);
+                    umma_commit_pair(st_empty + 8 * s);
+                    if (++s == GP_STAGES) { s = 0; phase ^= 1u; }
+                }
+                if (ok) umma_commit_pair(acc_full);
+            }
+            if (!ok) {
+                atomicCAS(p.err, 0, 0x30012);
+                *s_dead = 1;
+            }
+        }
+        __syncwarp();
+    } else if (warp == GP_LOADER) {
+        const size_t pitch = (size_t)p.M / 2;
+        const int row = lane >> 2, ch = lane & 3;   // 16 bytes of every eighth row
+        int s = 0;
+        uint32_t phase = 0;
+        bool ok = true, wrapped = false;
+        for (int item = first; item < items && ok; item += step) {
+            const PairItem w = pair_item(p, item);
+            const int block = 2 * w.tile_m + rank;
+            const uint8_t* src = p.packed + ((size_t)w.kb_lo * GM_BK + row) * pitch + (size_t)block * 64 + ch * 16;
+            for (int kb = 0; kb < w.n_kb; ++kb) {
+                if (wrapped) ok = __all_sync(0xffffffffu, *s_dead == 0 && mbar_wait(pk_empty + 8 * s, phase ^ 1u));
+                if (!ok) break;
+                if (block < p.Mb) {
+                    const uint32_t dst = smem_u32(pk_st + s * GP_PK_BYTES) + ch * 16;
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)   // the rows of an odd eight lie swapped in pairs
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;"
+                                     ::"r"(dst + (uint32_t)((8 * q + (row ^ (q & 1))) * 64)), "l"(src + (size_t)(8 * q) * pitch) : "memory");
+                }
+                src += (size_t)GM_BK * pitch;
+                asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(pk_full + 8 * s) : "memory");
+                if (++s == GP_PK_STAGES) { s = 0; phase ^= 1u; wrapped = true; }
+            }
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        if (!ok) {
+            if (lane == 0) atomicCAS(p.err, 0, 0x30015);
+            *s_dead = 1;
+        }
+        __syncwarp();
+    } else {
+        const int grp = (warp - 2) >> 2;
+        const int ut = (tid - 64) & 127, c = ut & 15, kc = ut >> 4;   // 8 outputs 8c.., 8 inputs 8kc.. of a K block
+        const int d_step = p.Mb % p.Kb;
+        // this thread's word of row 8 kc of a packed K block; the swap keeps the two kc of a warp off each other's banks
+        const uint32_t* pk_thr = reinterpret_cast<const uint32_t*>(pk_st + kc * 512 + c * 4);
+        const int pk_swap = kc & 1;
+        const uint32_t a_thr = (uint32_t)(c * 128 + ((kc ^ (c & 7)) << 4));
+        int s = grp, lap = 0;   // stage and lap of this group's next K block
+        int ps = grp;           // its place in the packed ring (a multiple of the groups: the laps of a group's places agree)
+        uint32_t pphase = 0;
+        int kb = grp, n = 0;
+        bool dead = false;
+        PairItem w = pair_item(p, first);
+        for (int item = first; item < items; item += step, ++n) {
+            const int block = 2 * w.tile_m + rank, ibk = block % p.Kb;
+            const bool valid = block < p.Mb;
+            DqConst ku = {0u, 0u, 0u};
+            if (UNIFORM) {
+                const uint32_t e = tab[ibk];
+                ku = make_const<EXACT>(__ushort_as_half((unsigned short)e), __ushort_as_half((unsigned short)(e >> 16)));
+            }
+            for (; kb < w.n_kb; kb += GP_GROUPS) {   // this group's K blocks of the item
+                bool ok = mbar_wait(pk_full + 8 * ps, pphase);
+                uint32_t cur[8];
+#pragma unroll
+                for (int r = 0; r < 8; ++r) cur[r] = pk_thr[ps * (GP_PK_BYTES / 4) + (r ^ pk_swap) * 16];
+                __syncwarp();
+                if (lane == 0) mbar_arrive(pk_empty + 8 * ps);
+                ps += GP_GROUPS;
+                if (ps >= GP_PK_STAGES) { ps -= GP_PK_STAGES; pphase ^= 1u; }
+                ok = ok && (lap == 0 || mbar_wait(st_empty + 8 * s, (uint32_t)(lap - 1) & 1u));
+                if (!__all_sync(0xffffffffu, ok && *s_dead == 0)) {
+                    if (lane == 0) atomicCAS(p.err, 0, 0x30013);
+                    *s_dead = 1;
+                    dead = true;
+                    break;
+                }
+                if (valid) {
+                    uint8_t* dst = a_st + s * GM_A_BYTES + a_thr;
+                    DqConst kq[4];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) kq[q] = ku;
+                    if (!UNIFORM) {   // the group moves by d_step from one input to the next
+                        const int j = (w.kb_lo + kb) * GM_BK + kc * 8;
+                        int g = (ibk + (j % p.Kb) * d_step) % p.Kb;
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            const uint32_t e0 = tab[g];
+                            g += d_step;
+                            g -= g >= p.Kb ? p.Kb : 0;
+                            const uint32_t e1 = tab[g];
+                            g += d_step;
+                            g -= g >= p.Kb ? p.Kb : 0;
+                            const DqConst k0 = make_const<EXACT>(__ushort_as_half((unsigned short)e0), __ushort_as_half((unsigned short)(e0 >> 16)));
+                            const DqConst k1 = make_const<EXACT>(__ushort_as_half((unsigned short)e1), __ushort_as_half((unsigned short)(e1 >> 16)));
+                            kq[q].z = prmt(k0.z, k1.z, 0x5410);
+                            kq[q].hz = prmt(k0.hz, k1.hz, 0x5410);
+                            kq[q].s = prmt(k0.s, k1.s, 0x5410);
+                        }
+                    }
+#pragma unroll
+                    for (int b = 0; b < 4; ++b) {   // outputs 2b and 2b + 1
+                        uint32_t lo[4], hi[4];
+#pragma unroll
+                        for (int q = 0; q < 4; ++q)
+                            dq_pair<EXACT>(prmt(cur[2 * q], cur[2 * q + 1], (uint32_t)(b | b << 4 | (4 + b) << 8 | (4 + b) << 12)), kq[q], lo[q], hi[q]);
+                        *reinterpret_cast<uint4*>(dst + (2 * b) * 2048) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+                        *reinterpret_cast<uint4*>(dst + (2 * b + 1) * 2048) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+                    }
+                }
+                // generic-proxy writes of A must be visible to the tensor core (async proxy) before the arrive
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive_leader(a_full + 8 * s);
+                s += GP_GROUPS;
+                if (s >= GP_STAGES) { s -= GP_STAGES; ++lap; }
+            }
+            // ---- epilogue: accumulators -> staging -> Y
+            if (!dead && !mbar_wait(acc_full, (uint32_t)n & 1u)) {
+                if (lane == 0) atomicCAS(p.err, 0, 0x30014);
+                *s_dead = 1;
+                dead = true;
+            }
+            __syncwarp();
+            dead = group_any(1 + grp, dead);   // the four warps meet in the staging tile: they go on, or leave, together
+            if (dead) break;
+            tc_fence_after();
+            const int q = warp & 3, m = 32 * q + lane;
+            __half* sg = reinterpret_cast<__half*>(stg + grp * GP_STG_BYTES);
+            const int i_local = 8 * (m & 15) + (m >> 4);
+            for (int c0 = 16 * grp; c0 < p.n_tile; c0 += 16 * GP_GROUPS) {
+                const int r0 = w.tile_n * p.n_tile + c0;
+                if (r0 >= p.rows) break;       // uniform over the group
+                uint32_t v[16];
+                float f[16];
+                tmem_ld16(tmem_base + ((uint32_t)(32 * q) << 16) + (uint32_t)c0, v);
+#pragma unroll
+                for (int e = 0; e < 16; ++e) f[e] = __uint_as_float(v[e]);
+                tmem_ld16(tmem_base + ((uint32_t)(32 * q) << 16) + (uint32_t)(GP_MAX_N + c0), v);
+#pragma unroll
+                for (int e = 0; e < 16; ++e) f[e] += __uint_as_float(v[e]);
+                if (!valid) continue;
+                if (w.slot >= 0) {
+                    float* dst = p.part + ((size_t)w.slot * p.n_tile + c0) * 256 + rank * 128 + m;
+#pragma unroll
+                    for (int e = 0; e < 16; ++e) dst[(size_t)e * 256] = f[e];
+                    continue;
+                }
+#pragma unroll
+                for (int e = 0; e < 16; ++e) {
+                    const __half h = __float2half_rn(f[e]);
+                    sg[e * GP_STG_LD + i_local] = p.epilogue == QW3_EPI_GELU ? gelu_h(h) : h;
+                }
+                named_barrier(1 + grp, 128);
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    const int piece = ut + 128 * k, e = piece >> 4, o8 = piece & 15;
+                    if (r0 + e < p.rows) {
+                        uint4 o = *reinterpret_cast<const uint4*>(sg + e * GP_STG_LD + o8 * 8);
+                        uint4* dst = reinterpret_cast<uint4*>(p.y + (size_t)(r0 + e) * p.M + (size_t)block * 128 + o8 * 8);
+                        if (p.epilogue == QW3_EPI_RESIDUAL) {
+                            const uint4 old = *dst;
+                            o = make_uint4(h2_add(old.x, o.x), h2_add(old.y, o.y), h2_add(old.z, o.z), h2_add(old.w, o.w));
+                        }
+                        *dst = o;
+                    }
+                }
+                named_barrier(1 + grp, 128);
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_leader(acc_empty);
+            kb = (kb - w.n_kb) & (GP_GROUPS - 1);   // first own K block of the next item
+            if (item + step < items) w = pair_item(p, item + step);
+        }
+    }
+    // nothing arrives at a CTA that has left: the producers and the epilogue warps have waited for every commit of their CTA
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512) : "memory");
+    }
+}
+
+// Sums the partial products of the split tiles in split order, rounds once to fp16 and stores two outputs a thread.
+__global__ void __launch_bounds__(256) gemm_pair_reduce_kernel(const PairParams p) {
+    const int tile = p.full + blockIdx.x, r = blockIdx.y * 2 + (threadIdx.x >> 7);
+    const int row = (tile % p.n_tiles_n) * p.n_tile + r, i = (threadIdx.x & 127) * 2, out = (tile / p.n_tiles_n) * 256 + i;
+    if (row >= p.rows || out >= p.M) return;
+    const int at = (i & 128) + 16 * (i & 7) + ((i & 127) >> 3);   // A's row of output i; output i + 1 is 16 rows on
+    const float* src = p.part + ((size_t)blockIdx.x * p.splits * p.n_tile + r) * 256 + at;
+    float a = src[0], b = src[16];
+#pragma unroll 4
+    for (int z = 1; z < p.splits; ++z) {
+        src += (size_t)p.n_tile * 256;
+        a += src[0];
+        b += src[16];
+    }
+    __half2* dst = reinterpret_cast<__half2*>(p.y + (size_t)row * p.M + out);
+    const __half2 old = p.epilogue == QW3_EPI_RESIDUAL ? *dst : __half2();
+    *dst = __halves2half2(gemm_epilogue(a, p.epilogue, __low2half(old)), gemm_epilogue(b, p.epilogue, __high2half(old)));
+}
+
 // ---------------------------------------------------------------------------------------------
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -359,6 +787,95 @@ static int encode_rows(CUtensorMap* map, const void* x, int64_t rows, int64_t K,
     return encode_f16_map(map, x, 2, dims, strides, box);
 }
 
+// How rows x M x K is cut for the pair kernel: the width of a row tile and the K splits of the tiles that do not fill a wave of
+// pairs.  The estimate counts K blocks: an MMA step of n_tile rows takes 2 n_tile cycles, and a K block is never cheaper than
+// its unpacking; a split tile pays for its partial products and the second kernel.
+struct PairCut { int n_tile, full, splits, items; };
+static PairCut pair_cut(long long rows, int M, int K, int pairs) {
+    const int n_kb = K / GM_BK, tiles_m = (M + 255) / 256;
+    PairCut best = {};
+    double best_cost = 0.0;
+    for (int n = 32; n <= GP_MAX_N; n += 32) {
+        if (n < GP_MAX_N && n * 2 <= rows && n < 160) continue;   // narrow tiles only where few of them cover the rows
+        const long long tiles = tiles_m * ((rows + n - 1) / n);
+        const double kb_cost = n > 128 ? 2.0 * n : 256.0;
+        const int tail = (int)(tiles % pairs);
+        const long long waves = tiles / pairs;
+        for (int z = 1; z <= 16 && n_kb / z >= 8; ++z) {
+            if (z > 1 && (tail == 0 || (long long)tail * z * n > (long long)(WS_PARTIALS / 256))) break;
+            const int tail_waves = (tail * z + pairs - 1) / pairs;
+            const double cost = waves * (n_kb * kb_cost + 2000.0) + tail_waves * ((n_kb + z - 1) / z * kb_cost + 2000.0) + (z > 1 ? 6000.0 : 0.0);
+            if (best.n_tile == 0 || cost < best_cost) {
+                best_cost = cost;
+                best.n_tile = n;
+                best.full = (int)(z > 1 ? tiles - tail : tiles);
+                best.splits = z;
+                best.items = best.full + (z > 1 ? tail * z : 0);
+            }
+        }
+    }
+    return best;
+}
+
+// Where the pairs are the faster kernel (us, one-CTA kernel / pairs).  More than 128 rows: 12288 x 4096 34.9 / 26.8 at 160 rows and
+// 202 / 156 at 2048, 4096 x 12288 79.5 / 65.9 at 512 rows; but where neither a single wave nor a split of the last one
+// fills the chip the smaller tiles win (4096 x 12288 at 2048 rows 175 / 208).  Up to 128 rows a call is short and the pairs' start
+// and second kernel show (4096 x 4096 at 64 rows 16.4 / 20.6), unless there are 256-output tiles for every pair of SMs
+// (151936 x 4096 at 64 rows 251 / 190).  The result is stored by 16 bytes; an item has two K blocks for each unpack group.
+static bool pair_wanted(const W4Desc* d, long long rows, const void* d_y, const Workspace* ws) {
+    const int pairs = ws->sm_count / 2;
+    if (d->K / GM_BK < 2 * GP_GROUPS || pairs < 1 || (reinterpret_cast<uintptr_t>(d_y) & 15) != 0) return false;
+    if (rows <= 128) return (d->M + 255) / 256 >= pairs;
+    const PairCut cut = pair_cut(rows, (int)d->M, (int)d->K, pairs);
+    return cut.splits > 1 || cut.items <= pairs;
+}
+
+static int pair_launch(const W4Desc* d, const void* d_x, long long rows, void* d_y, const Workspace* ws, cudaStream_t st, int epilogue) {
+    PairParams p = {};
+    p.packed = d->packed;
+    p.scale = d->scale; p.zp = d->zp; p.n_alloc = (int)d->n_alloc;
+    p.M = (int)d->M; p.K = (int)d->K; p.Mb = p.M / 128; p.Kb = p.K / 128;
+    p.rows = (int)rows;
+    const int pairs = ws->sm_count / 2;
+    const PairCut cut = pair_cut(rows, p.M, p.K, pairs);
+    p.n_tile = cut.n_tile; p.full = cut.full; p.splits = cut.splits; p.items = cut.items;
+    p.n_tiles_m = (p.M + 255) / 256;
+    p.n_tiles_n = (int)((rows + p.n_tile - 1) / p.n_tile);
+    p.epilogue = epilogue;
+    p.y = static_cast<__half*>(d_y);
+    p.part = ws->partials;
+    p.err = ws->err;
+    CUtensorMap tmap_x;
+    const int rc = encode_rows(&tmap_x, d_x, rows, d->K, p.n_tile / 2);
+    if (rc != QW3_OK) return rc;
+    static std::once_flag attr_once[16];
+    int dev = 0;
+    QW3_CUDA(cudaGetDevice(&dev));
+    auto set_attr = [] {
+        cudaFuncSetAttribute(gemm_w4a16_pair_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GP_SMEM);
+        cudaFuncSetAttribute(gemm_w4a16_pair_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GP_SMEM);
+        cudaFuncSetAttribute(gemm_w4a16_pair_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GP_SMEM);
+        cudaFuncSetAttribute(gemm_w4a16_pair_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GP_SMEM);
+    };
+    if (dev < 16) std::call_once(attr_once[dev], set_attr);
+    else set_attr();
+    const unsigned grid = 2u * (unsigned)(p.items < pairs ? p.items : pairs);
+    if (d->zp_integral) {
+        if (d->uniform) gemm_w4a16_pair_kernel<true, true><<<grid, GP_THREADS, GP_SMEM, st>>>(tmap_x, p);
+        else gemm_w4a16_pair_kernel<true, false><<<grid, GP_THREADS, GP_SMEM, st>>>(tmap_x, p);
+    } else {
+        if (d->uniform) gemm_w4a16_pair_kernel<false, true><<<grid, GP_THREADS, GP_SMEM, st>>>(tmap_x, p);
+        else gemm_w4a16_pair_kernel<false, false><<<grid, GP_THREADS, GP_SMEM, st>>>(tmap_x, p);
+    }
+    QW3_CUDA(cudaGetLastError());
+    if (p.splits > 1) {
+        const dim3 g((unsigned)(p.n_tiles_m * p.n_tiles_n - p.full), (unsigned)(p.n_tile / 2));
+        gemm_pair_reduce_kernel<<<g, 256, 0, st>>>(p);
+        QW3_CUDA(cudaGetLastError());
+    }
+    return QW3_OK;
+}
+
 }  // namespace qw3
 
 using namespace qw3;
@@ -378,6 +895,8 @@ int qw3::gemm_launch(qw3_w4_t w, const void* d_x, int64_t rows, void* d_y, qw3_w
     QW3_REQUIRE(rows >= 1 && rows <= (1 << 20), "qw3_gemm_w4a16: rows out of range");
     QW3_REQUIRE((reinterpret_cast<uintptr_t>(d_x) & 15) == 0, "qw3_gemm_w4a16: X must be 16-byte aligned");
     const W4Desc* d = w4_desc(w);
+    if (pair_wanted(d, rows, d_y, ws_struct(ws)))
+        return pair_launch(d, d_x, rows, d_y, ws_struct(ws), static_cast<cudaStream_t>(stream), epilogue);
     GemmParams p = {};
     p.packed = d->packed;
     p.scale = d->scale; p.zp = d->zp; p.n_alloc = (int)d->n_alloc;
@@ -410,7 +929,7 @@ int qw3::gemm_launch(qw3_w4_t w, const void* d_x, int64_t rows, void* d_y, qw3_w
     // Few rows and few output tiles leave most SMs without a CTA: split K over grid.z (fp32 partial products in the
     // workspace, summed in split order by a second kernel) until ~one CTA per SM, while the partials fit.
     const long long ctas = (d->M / GM_TILE_M) * ((rows + p.n_tile - 1) / p.n_tile);
-    const long long part_cap = (long long)(WS_MAX_CTAS + WS_MAX_TILES) * WS_TILE;   // floats in the workspace
+    const long long part_cap = (long long)WS_PARTIALS;   // floats in the workspace
     int splits = 1;
     while (splits < 8 && ctas * (splits * 2) <= ws_struct(ws)->sm_count && (p.K / GM_BK) / (splits * 2) >= 8 &&
            (long long)(splits * 2) * rows * d->M <= part_cap)

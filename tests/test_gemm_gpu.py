@@ -77,3 +77,29 @@ def test_gemm_sweep_rows_equal_gemv(ops, orc, cuda, M, K, R):
         # one-ulp differences only; their share grows with the number of accumulation steps (K)
         assert ((d <= 1) | near).all() and (d > 0).mean() < (0.05 if K <= 4096 else 0.08)
     ws.check()
+
+
+@pytest.mark.parametrize("M,K,R,integral", [
+    (384, 512, 130, True),     # an odd number of 128-output blocks: the last pair has one CTA without outputs; fewest K blocks
+    (256, 640, 161, True),     # K blocks that are no multiple of the rings and of the unpack groups
+    (640, 1152, 159, False), (2176, 896, 160, True), (896, 2176, 193, False),   # group depends on the input, K not a power of two
+    (4096, 512, 257, True), (1664, 1536, 129, True),                           # one row past a row tile
+    (19200, 4096, 160, False),   # more tiles than pairs of SMs: a whole wave, then a tile whose K is split
+    (256, 8192, 144, True)])     # one tile: K split over many pairs
+def test_gemm_pairs_edges(ops, orc, cuda, M, K, R, integral):
+    p, s, z = orc.gen_linear(43, M, K)
+    if not integral:
+        z = orc.gen_normal_f16(43, 999, M // 128, 7.5, 1.3)
+    X = orc.gen_normal_f16(43, orc.ACT, R * K).reshape(R, K)
+    got, w, ws = _gemm(ops, cuda, p, s, z, M, K, X, zp_integral=integral)
+    rows = sorted(set([0, 1, R // 2, R - 2, R - 1]))
+    y32, y16 = orc.gemm_w4a16(p, s, z, M, K, X[rows])
+    _check(got[rows], y32, y16, f"{M}x{K} rows {R}", differ=0.05 if K <= 4096 else 0.08)
+    # a result that does not start on 16 bytes takes the one-CTA kernel
+    off = torch.zeros(R * M + 8, dtype=torch.float16, device=cuda)
+    y = off[2:2 + R * M].view(R, M)
+    ops.gemm_w4a16(w, ws, _to_dev(X, cuda), y)
+    ws.check()
+    d = _ulp_diff(y.cpu().numpy(), got)
+    near = np.abs(y.cpu().numpy().astype(np.float32) - got.astype(np.float32)) <= 1e-4 * np.abs(y32).mean()
+    assert ((d <= 1) | near).all() and (d > 0).mean() < 0.08
