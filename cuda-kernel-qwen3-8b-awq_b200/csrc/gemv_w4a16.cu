@@ -451,7 +451,7 @@ int encode_2d_u32(CUtensorMap* map, const void* base, uint64_t inner_elems, uint
 
 size_t workspace_bytes() {
     size_t b = 0;
-    b += (size_t)(WS_MAX_CTAS + WS_MAX_TILES) * WS_TILE * 4;  // partials
+    b += WS_PARTIALS * 4;  // partials
     b += (size_t)WS_MAX_TILES * 4;                            // counters
     b += 256;                                                 // tiles_done
     b += (size_t)WS_MAX_TILES * 4 * 2;                        // arg_val, arg_idx
@@ -463,7 +463,7 @@ size_t workspace_bytes() {
 
 void workspace_carve(Workspace* ws, void* base) {
     uint8_t* p = static_cast<uint8_t*>(base);
-    ws->partials = reinterpret_cast<float*>(p);   p += (size_t)(WS_MAX_CTAS + WS_MAX_TILES) * WS_TILE * 4;
+    ws->partials = reinterpret_cast<float*>(p);   p += WS_PARTIALS * 4;
     ws->counters = reinterpret_cast<int32_t*>(p); p += (size_t)WS_MAX_TILES * 4;
     ws->tiles_done = reinterpret_cast<int32_t*>(p); p += 256;
     ws->arg_val = reinterpret_cast<float*>(p);    p += (size_t)WS_MAX_TILES * 4;
@@ -474,7 +474,7 @@ void workspace_carve(Workspace* ws, void* base) {
 }
 
 // Byte offset (within the workspace allocation) from which everything must start at zero.
-static size_t workspace_zero_from() { return (size_t)(WS_MAX_CTAS + WS_MAX_TILES) * WS_TILE * 4; }
+static size_t workspace_zero_from() { return WS_PARTIALS * 4; }
 
 static size_t gemv_smem_bytes(int K, bool uniform) {
     size_t b = (size_t)NSTAGES * STAGE_BYTES + RED_BYTES + (size_t)K * 2;
@@ -674,7 +674,10 @@ int gemv_launch(const W4Desc* d, const Qw3GemvArgs* a, const Workspace* ws, bool
     const size_t smem = gemv_smem_bytes(p.K, uniform);
     QW3_REQUIRE(smem <= 227 * 1024, "qw3_gemv_w4a16: in_dim=%d needs %zu bytes of shared memory", p.K, smem);
     int grid = ws->sm_count < WS_MAX_CTAS ? ws->sm_count : WS_MAX_CTAS;
-    if ((long long)grid > p.U) grid = (int)p.U;
+    // A stage of 64 rows keeps all sixteen consumer warps of a CTA busy at once: a CTA with less than one is no faster and
+    // leaves one more set of partial sums to add (1536 x 512: 16 CTAs instead of 128).
+    const long long stages = (p.U + STAGE_UNITS - 1) / STAGE_UNITS;
+    if (grid > stages) grid = (int)stages;
     if (uniform) {
         if (d->zp_integral) return launch_gemv<true, true>(d, p, grid, smem, pdl, st);
         return launch_gemv<true, false>(d, p, grid, smem, pdl, st);
