@@ -173,7 +173,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
         const int pos_first = pos - lane;                                      // of the warp's first row
         const float c = (float)(1.4426950408889634 / 11.313708498984761);      // log2(e) / sqrt(128), Inference.cu:218
         float m = -INFINITY, mc = 0.0f, l = 0.0f;   // m: maximum in use (raw scores), mc = m c
-        bool ok = true;
+        float mr = 0.0f;                            // m c - mc where that is not small
+        bool coarse = false, ok = true;             // some row of the warp has mr
         for (int j = 0; j < n_tiles && ok; ++j) {
             const int b = j & 1;
             ok = __all_sync(0xffffffffu, *s_dead == 0 && mbar_wait(s_full + 16 * t + 8 * b, (uint32_t)(j >> 1) & 1u));
@@ -197,7 +198,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
             const float mt = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
             if (__any_sync(0xffffffffu, (mt - m) * c > 8.0f)) {   // rare after the first tile
                 const float mn = fmaxf(m, mt), nmc = mn == -INFINITY ? 0.0f : mn * c;
-                const float f = m == -INFINITY ? 0.0f : ex2(mc - nmc);
+                const float nmr = fabsf(nmc) >= 1048576.0f ? fmaf(mn, c, -nmc) : 0.0f;
+                const float f = m == -INFINITY ? 0.0f : ex2((mc - nmc) + (mr - nmr));
                 if (j > 0) {
                     ok = __all_sync(0xffffffffu, mbar_wait(pv_done + 16 * t + 8 * (b ^ 1), (uint32_t)((j - 1) >> 1) & 1u));
                     if (!ok) break;
@@ -215,6 +217,15 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
                 l *= f;
                 m = mn;
                 mc = nmc;
+                mr = nmr;
+                coarse = __any_sync(0xffffffffu, mr != 0.0f);
+            }
+            float sc = c, off = mc;
+            if (coarse) {
+#pragma unroll
+                for (int e = 0; e < 64; ++e) s[e] = fmaf(s[e], c, -mc) - mr;
+                sc = 1.0f;
+                off = 0.0f;
             }
             float ls[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
@@ -222,7 +233,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
                 uint32_t hi[16], lo[16];
 #pragma unroll
                 for (int e = 0; e < 16; ++e) {
-                    const float a0 = ex2(fmaf(s[32 * h + 2 * e], c, -mc)), a1 = ex2(fmaf(s[32 * h + 2 * e + 1], c, -mc));
+                    const float a0 = ex2(fmaf(s[32 * h + 2 * e], sc, -off)), a1 = ex2(fmaf(s[32 * h + 2 * e + 1], sc, -off));
                     ls[(2 * e) & 3] += a0;
                     ls[(2 * e + 1) & 3] += a1;
                     const __half2 hh = __floats2half2_rn(a0, a1);

@@ -89,6 +89,25 @@ def test_attention_prefill_pairs_of_row_tiles(ops, orc, cuda, heads, max_pos, po
         assert (_ulp_diff(got[r], want) > 1).mean() < 0.01, r
 
 
+@pytest.mark.parametrize("gain", [1000.0, 4000.0, 15000.0])
+def test_attention_prefill_large_scores(ops, orc, cuda, gain):
+    """Rows and keys of the size fp16 can hold, every row equal to one of its keys: scores of 1e7 to 3e9, where a row's maximum
+    times log2(e) / sqrt(128) has no fraction left in fp32.  The equal key wins by far, so the result is its value row."""
+    heads, max_pos, pos0, rows = 2, 512, 100, 300
+    qkv = orc.gen_normal_f16(33, orc.ACT, rows * 3 * heads * 128).reshape(rows, 3 * heads * 128).copy()
+    kc = orc.gen_normal_f16(33, orc.KV_K, heads * max_pos * 128).astype(np.float32).clip(-4, 4).reshape(heads, max_pos, 128)
+    kc = (kc * gain).astype(np.float16)
+    vc = orc.gen_normal_f16(33, orc.KV_V, heads * max_pos * 128).reshape(heads, max_pos, 128)
+    key = np.array([(37 * r) % (pos0 + r + 1) for r in range(rows)])
+    for h in range(heads):
+        qkv[:, 128 * h:128 * h + 128] = kc[h, key]
+    got = ops.attn_prefill(_to_dev(qkv, cuda), _to_dev(kc.ravel(), cuda), _to_dev(vc.ravel(), cuda), heads, max_pos, pos0, rows).cpu().numpy()
+    for r in (0, 63, 128, 299):
+        want = orc.attention(np.ascontiguousarray(qkv[r, :heads * 128]), kc.ravel(), vc.ravel(), heads, 128, max_pos, pos0 + r + 1)
+        assert np.array_equal(want.reshape(heads, 128), vc[:, key[r]]), r
+    for h in range(heads):
+        assert np.array_equal(got[:, 128 * h:128 * h + 128], vc[h, key])
+
 
 def test_embed_gather_bit_exact(ops, orc, cuda):
     H, V = 512, 4096 + 256
