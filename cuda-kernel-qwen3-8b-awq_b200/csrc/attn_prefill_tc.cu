@@ -35,9 +35,57 @@ __device__ __forceinline__ float ex2(float x) {
 }
 
 struct AttnParams {
+    const __half* qkv;
+    const __half* kc;
+    const __half* vc;
+    long long max_pos;
     __half* ctx;
     int hidden, pos0, rows;
 };
+
+// One row by a warp, from global memory and in 32-bit arithmetic: rows whose tile holds Inf or NaN in V behind the row.  The tensor
+// cores multiply these by the zeros of the masked probabilities, and the sum is NaN; here nothing past the row's last key is read.
+__device__ __noinline__ void attn_row(const __half* q, const __half* k, const __half* v, int n_keys, __half* dst, int lane) {
+    float m = -INFINITY, l = 0.0f, o[4] = {0.0f, 0.0f, 0.0f, 0.0f};   // outputs 4 lane .. 4 lane + 3
+    for (int k0 = 0; k0 < n_keys; k0 += 32) {
+        float s = -INFINITY;
+        if (k0 + lane < n_keys) {
+            const uint4* kr = reinterpret_cast<const uint4*>(k + (size_t)(k0 + lane) * 128);
+            const uint4* qr = reinterpret_cast<const uint4*>(q);
+            s = 0.0f;
+            for (int i = 0; i < 16; ++i) {
+                const uint4 a = qr[i], b = kr[i];
+                const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, bw[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const float2 x = __half22float2(*reinterpret_cast<const __half2*>(&aw[e])), y = __half22float2(*reinterpret_cast<const __half2*>(&bw[e]));
+                    s = fmaf(x.y, y.y, fmaf(x.x, y.x, s));
+                }
+            }
+            s *= 1.0f / sqrtf(128.0f);   // Inference.cu:218
+        }
+        float mn = fmaxf(m, s);
+        for (int d = 16; d > 0; d >>= 1) mn = fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, d));
+        const float f = m == -INFINITY ? 0.0f : expf(m - mn), pr = s == -INFINITY ? 0.0f : expf(s - mn);
+        m = mn;
+        l = l * f + pr;   // this lane's keys
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[e] *= f;
+        for (int j = 0; j < 32 && k0 + j < n_keys; ++j) {
+            const float pj = __shfl_sync(0xffffffffu, pr, j);
+            const uint2 w = *reinterpret_cast<const uint2*>(v + (size_t)(k0 + j) * 128 + 4 * lane);
+            const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&w.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&w.y));
+            o[0] = fmaf(pj, a.x, o[0]);
+            o[1] = fmaf(pj, a.y, o[1]);
+            o[2] = fmaf(pj, b.x, o[2]);
+            o[3] = fmaf(pj, b.y, o[3]);
+        }
+    }
+    for (int d = 16; d > 0; d >>= 1) l += __shfl_xor_sync(0xffffffffu, l, d);
+    __half2* out = reinterpret_cast<__half2*>(dst + 4 * lane);
+    out[0] = __floats2half2_rn(o[0] / l, o[1] / l);
+    out[1] = __floats2half2_rn(o[2] / l, o[3] / l);
+}
 
 __global__ void __launch_bounds__(AT_THREADS, 1)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
@@ -257,6 +305,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
         tc_fence_after();
         __half* dst = p.ctx + (size_t)row * p.hidden + head * 128;
         const bool wide = (reinterpret_cast<uintptr_t>(p.ctx) & 15) == 0;   // the caller's ctx need only be aligned for pairs
+        float finite = 0.0f;   // NaN as soon as an output is NaN or Inf
 #pragma unroll
         for (int h = 0; h < 4; ++h) {
             uint32_t o[32];
@@ -269,7 +318,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
                     uint32_t w[4];
 #pragma unroll
                     for (int k = 0; k < 4; ++k) {   // one rounding to fp16, Inference.cu:257-265
-                        const __half2 v = __floats2half2_rn(__uint_as_float(o[e + 2 * k]) / l, __uint_as_float(o[e + 2 * k + 1]) / l);
+                        const float a = __uint_as_float(o[e + 2 * k]) / l, b = __uint_as_float(o[e + 2 * k + 1]) / l;
+                        const __half2 v = __floats2half2_rn(a, b);
+                        finite = fmaf(a, 0.0f, fmaf(b, 0.0f, finite));
                         w[k] = ok ? *reinterpret_cast<const uint32_t*>(&v) : 0x7fff7fffu;
                     }
                     if (wide) {
@@ -280,6 +331,13 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
                     }
                 }
             }
+        }
+        __syncwarp();   // a row that is done again has been stored
+        for (uint32_t redo = ok ? __ballot_sync(0xffffffffu, row < p.rows && finite != 0.0f) : 0u; redo != 0; redo &= redo - 1) {
+            const int r = row - lane + __ffs(redo) - 1;
+            const size_t at = (size_t)head * p.max_pos * 128;
+            attn_row(p.qkv + (size_t)r * 3 * p.hidden + head * 128, p.kc + at, p.vc + at, p.pos0 + r + 1,
+                     p.ctx + (size_t)r * p.hidden + head * 128, lane);
         }
     }
     tc_fence_before();
@@ -309,7 +367,8 @@ int attn_prefill_tc_launch(const void* qkv, const void* kc, const void* vc, int 
     auto set_attr = [] { cudaFuncSetAttribute(attn_prefill_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AT_SMEM); };
     if (dev >= 0 && dev < 64) std::call_once(attr_once[dev], set_attr);
     else set_attr();
-    AttnParams p = {static_cast<__half*>(ctx), hidden, pos0, rows};
+    AttnParams p = {static_cast<const __half*>(qkv), static_cast<const __half*>(kc), static_cast<const __half*>(vc), max_pos,
+                    static_cast<__half*>(ctx), hidden, pos0, rows};
     attn_prefill_tc_kernel<<<dim3(heads, (rows + 2 * AT_ROWS - 1) / (2 * AT_ROWS)), AT_THREADS, AT_SMEM, st>>>(tm_q, tm_k, tm_v, p);
     QW3_CUDA(cudaGetLastError());
     return QW3_OK;

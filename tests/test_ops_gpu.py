@@ -109,6 +109,28 @@ def test_attention_prefill_large_scores(ops, orc, cuda, gain):
         assert np.array_equal(got[:, 128 * h:128 * h + 128], vc[h, key])
 
 
+@pytest.mark.parametrize("heads,max_pos,pos0,rows,at,value", [(2, 512, 100, 300, 200, np.inf), (1, 384, 0, 256, 255, np.nan), (1, 700, 63, 40, 33, -np.inf),
+                                                              (2, 300, 7, 129, 1, np.nan)])
+def test_attention_prefill_nothing_behind_a_row_reaches_it(ops, orc, cuda, heads, max_pos, pos0, rows, at, value):
+    """Inf or NaN in one value row of the block itself, and in its key row: rows before it are those of finite caches."""
+    H = heads * 128
+    qkv = orc.gen_normal_f16(34, orc.ACT, rows * 3 * H).reshape(rows, 3 * H)
+    kc = orc.gen_normal_f16(34, orc.KV_K, heads * max_pos * 128).reshape(heads, max_pos, 128).copy()
+    vc = orc.gen_normal_f16(34, orc.KV_V, heads * max_pos * 128).reshape(heads, max_pos, 128).copy()
+    kc[0, pos0 + at, 3] = value
+    vc[0, pos0 + at, [5, 77]] = value
+    got = ops.attn_prefill(_to_dev(qkv, cuda), _to_dev(kc.ravel(), cuda), _to_dev(vc.ravel(), cuda), heads, max_pos, pos0, rows).cpu().numpy()
+    finite = np.isfinite(got)
+    assert finite[:at].all() and finite[:, 128:].all() and not finite[at:, [5, 77]].any()
+    for r in sorted(set([0, 1, at - 64, at - 1, at, at + 1, rows - 1]) & set(range(rows))):
+        want = orc.attention(np.ascontiguousarray(qkv[r, :H]), kc.ravel(), vc.ravel(), heads, 128, max_pos, pos0 + r + 1)
+        ok = np.isfinite(want)
+        assert np.array_equal(ok, finite[r]), r
+        err = np.abs(got[r].astype(np.float32) - want.astype(np.float32))[ok]
+        assert (err <= 2e-2 * np.abs(want.astype(np.float32)[ok]) + 2e-3).all(), r
+        assert (_ulp_diff(got[r][ok], want[ok]) > 1).sum() <= 0.01 * ok.sum(), r
+
+
 def test_embed_gather_bit_exact(ops, orc, cuda):
     H, V = 512, 4096 + 256
     p, s, z = orc.gen_linear(24, H, V, kind=orc.EMB)
