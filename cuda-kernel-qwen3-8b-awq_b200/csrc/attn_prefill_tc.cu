@@ -15,7 +15,8 @@
 // 1953 rows at position 2048, 32 heads: 590 us with warp-level MMAs (mma.sync, 64 rows a CTA), 160 now, 0.36 of the measured bf16
 // rate in useful operations (the second term of P and the masked halves of the diagonal tiles are not counted).
 // Bound: the MMAs, 768 cycles per 128 x 64 scores (256 for S, 256 for each term of P), beside 512 cycles of exponentials.
-// All waits are bounded; after one that gives up the rows are written as NaN.
+// All waits are bounded.  After one that gives up the error word is set, rows that are not finished are written as NaN, and the CTA
+// leaves when its copies and MMAs in flight are done.
 #include <mutex>
 
 #include "tc05.cuh"
@@ -41,7 +42,10 @@ struct AttnParams {
     long long max_pos;
     __half* ctx;
     int hidden, pos0, rows;
+    int* err;   // null: the word below
 };
+// Error word of calls without a workspace, one on every GPU that loads the library.
+static __device__ int g_attn_err;
 
 // One row by a warp, from global memory and in 32-bit arithmetic: rows whose tile holds Inf or NaN in V behind the row.  The tensor
 // cores multiply these by the zeros of the masked probabilities, and the sum is NaN; here nothing past the row's last key is read.
@@ -87,6 +91,8 @@ __device__ __noinline__ void attn_row(const __half* q, const __half* k, const __
     out[1] = __floats2half2_rn(o[2] / l, o[3] / l);
 }
 
+// POLL_ONCE: a wait looks at its barrier once and gives up (qw3_attn_prefill_poll_once).
+template <bool POLL_ONCE>
 __global__ void __launch_bounds__(AT_THREADS, 1)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                        const __grid_constant__ CUtensorMap tm_v, const AttnParams p) {
@@ -97,9 +103,15 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
     uint64_t* bars = reinterpret_cast<uint64_t*>(v_s + AT_STAGES * AT_KV_BYTES);
     const uint32_t q_full = smem_u32(bars), k_full = q_full + 8, v_full = k_full + 8 * AT_STAGES, k_empty = v_full + 8 * AT_STAGES,
                    v_empty = k_empty + 8 * AT_STAGES, s_full = v_empty + 8 * AT_STAGES /* [tile][buffer] */, p_full = s_full + 32,
-                   pv_done = p_full + 32 /* [tile][buffer] */;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 1 + 4 * AT_STAGES + 12);
+                   pv_done = p_full + 32 /* [tile][buffer] */, drain = pv_done + 32;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 + 4 * AT_STAGES + 12);
     volatile int* s_dead = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+    const auto wait = [](uint32_t bar, uint32_t parity) { return POLL_ONCE ? mbar_poll(bar, parity) : mbar_wait(bar, parity); };
+    const auto give_up = [&](int code) {
+        atomicCAS(p.err != nullptr ? p.err : &g_attn_err, 0, code);
+        *s_dead = 1;
+    };
 
     const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
     const int head = blockIdx.x, r0 = (int)(gridDim.y - 1 - blockIdx.y) * 2 * AT_ROWS;   // the blocks with the most keys start first
@@ -108,6 +120,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
 
     if (tid == 0) {
         mbar_init(q_full, 1);
+        mbar_init(drain, 1);
         for (int s = 0; s < AT_STAGES; ++s) {
             mbar_init(k_full + 8 * s, 1);
             mbar_init(v_full + 8 * s, 1);
@@ -138,26 +151,34 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
             for (int t = 0; t < 2; ++t)
                 for (int h = 0; h < 2; ++h)
                     tma_load_2d(smem_u32(q_s + t * AT_Q_BYTES + h * (AT_Q_BYTES / 2)), &tm_q, head * 128 + 64 * h, r0 + AT_ROWS * t, q_full);
+            int issued[2] = {0, 0};   // tiles of K and V
             for (int j = 0; j < n_tiles && ok; ++j) {
                 const int s = j % AT_STAGES;
                 const uint32_t lap = (uint32_t)(j / AT_STAGES);
                 for (int kv = 0; kv < 2 && ok; ++kv) {
                     const uint32_t full = (kv ? v_full : k_full) + 8 * s, empty = (kv ? v_empty : k_empty) + 8 * s;
                     uint8_t* dst = (kv ? v_s : k_s) + s * AT_KV_BYTES;
-                    if (lap > 0) ok = mbar_wait(empty, (lap - 1) & 1u);
+                    if (lap > 0) ok = wait(empty, (lap - 1) & 1u);
                     if (*s_dead != 0) ok = false;
                     if (!ok) break;
                     mbar_expect_tx(full, AT_KV_BYTES);
                     for (int h = 0; h < 2; ++h)
                         tma_load_3d(smem_u32(dst + h * (AT_KV_BYTES / 2)), kv ? &tm_v : &tm_k, 64 * h, j * AT_KEYS, head, full);
+                    ++issued[kv];
                 }
             }
             // drain: the last release arrivals land before the CTA may leave
             for (int j = n_tiles < AT_STAGES ? 0 : n_tiles - AT_STAGES; j < n_tiles && ok; ++j) {
                 const uint32_t parity = (uint32_t)(j / AT_STAGES) & 1u;
-                ok = mbar_wait(k_empty + 8 * (j % AT_STAGES), parity) && mbar_wait(v_empty + 8 * (j % AT_STAGES), parity);
+                ok = wait(k_empty + 8 * (j % AT_STAGES), parity) && wait(v_empty + 8 * (j % AT_STAGES), parity);
             }
-            if (!ok) *s_dead = 1;
+            if (!ok) {
+                give_up(0x30021);
+                mbar_wait(q_full, 0);   // the copies in flight
+                for (int kv = 0; kv < 2; ++kv)
+                    for (int j = max(issued[kv] - AT_STAGES, 0); j < issued[kv]; ++j)
+                        mbar_wait((kv ? v_full : k_full) + 8 * (j % AT_STAGES), (uint32_t)(j / AT_STAGES) & 1u);
+            }
         }
         __syncwarp();
     } else if (warp == 1) {
@@ -176,9 +197,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
                              idesc_s, ks > 0 ? 1u : 0u);
                 umma_commit(s_full + 16 * t + 8 * (j & 1));
             };
-            bool ok = mbar_wait(q_full, 0);
+            bool ok = wait(q_full, 0);
             for (int j = 0; j < 2 && j < n_tiles && ok; ++j) {
-                ok = mbar_wait(k_full + 8 * j, 0);
+                ok = wait(k_full + 8 * j, 0);
                 if (!ok) break;
                 scores(0, j);
                 scores(1, j);
@@ -186,9 +207,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
             }
             for (int j = 0; j < n_tiles && ok; ++j) {
                 const int s = j % AT_STAGES, b = j & 1;
-                ok = *s_dead == 0 && mbar_wait(v_full + 8 * s, (uint32_t)(j / AT_STAGES) & 1u);
+                ok = *s_dead == 0 && wait(v_full + 8 * s, (uint32_t)(j / AT_STAGES) & 1u);
                 for (int t = 0; t < 2 && ok; ++t) {
-                    ok = mbar_wait(p_full + 16 * t + 8 * b, (uint32_t)(j >> 1) & 1u);
+                    ok = wait(p_full + 16 * t + 8 * b, (uint32_t)(j >> 1) & 1u);
                     if (!ok) break;
                     tc_fence_after();
                     const uint32_t a = tmem + 256 + 128 * t + 64 * b;
@@ -203,14 +224,16 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
                     // the next scores of the buffer: issued after, and so executed after, the product that reads P there
                     if (j + 2 < n_tiles) {
                         const int s2 = (j + 2) % AT_STAGES;
-                        if (t == 0) ok = mbar_wait(k_full + 8 * s2, (uint32_t)((j + 2) / AT_STAGES) & 1u);
+                        if (t == 0) ok = wait(k_full + 8 * s2, (uint32_t)((j + 2) / AT_STAGES) & 1u);
                         if (!ok) break;
                         scores(t, j + 2);
                         if (t == 1) umma_commit(k_empty + 8 * s2);
                     }
                 }
             }
-            if (!ok) *s_dead = 1;
+            if (!ok) give_up(0x30022);
+            umma_commit(drain);   // whoever gives up: the CTA does not leave before its MMAs are done
+            mbar_wait(drain, 0);
         }
         __syncwarp();
     } else if (warp >= 4) {
@@ -225,7 +248,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
         bool coarse = false, ok = true;             // some row of the warp has mr
         for (int j = 0; j < n_tiles && ok; ++j) {
             const int b = j & 1;
-            ok = __all_sync(0xffffffffu, *s_dead == 0 && mbar_wait(s_full + 16 * t + 8 * b, (uint32_t)(j >> 1) & 1u));
+            ok = __all_sync(0xffffffffu, *s_dead == 0 && wait(s_full + 16 * t + 8 * b, (uint32_t)(j >> 1) & 1u));
             if (!ok) break;
             tc_fence_after();
             uint32_t sr[64];
@@ -249,7 +272,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
                 const float nmr = fabsf(nmc) >= 1048576.0f ? fmaf(mn, c, -nmc) : 0.0f;
                 const float f = m == -INFINITY ? 0.0f : ex2((mc - nmc) + (mr - nmr));
                 if (j > 0) {
-                    ok = __all_sync(0xffffffffu, mbar_wait(pv_done + 16 * t + 8 * (b ^ 1), (uint32_t)((j - 1) >> 1) & 1u));
+                    ok = __all_sync(0xffffffffu, wait(pv_done + 16 * t + 8 * (b ^ 1), (uint32_t)((j - 1) >> 1) & 1u));
                     if (!ok) break;
                     tc_fence_after();
 #pragma unroll
@@ -300,8 +323,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
             if (lane == 0) mbar_arrive(p_full + 16 * t + 8 * b);
         }
         for (int j = n_tiles < 2 ? 0 : n_tiles - 2; j < n_tiles && ok; ++j)
-            ok = __all_sync(0xffffffffu, mbar_wait(pv_done + 16 * t + 8 * (j & 1), (uint32_t)(j >> 1) & 1u));
-        if (!ok) *s_dead = 1;
+            ok = __all_sync(0xffffffffu, wait(pv_done + 16 * t + 8 * (j & 1), (uint32_t)(j >> 1) & 1u));
+        if (!ok && lane == 0) give_up(0x30023);
+        __syncwarp();
         tc_fence_after();
         __half* dst = p.ctx + (size_t)row * p.hidden + head * 128;
         const bool wide = (reinterpret_cast<uintptr_t>(p.ctx) & 15) == 0;   // the caller's ctx need only be aligned for pairs
@@ -350,7 +374,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
 
 // qkv [rows][3 * hidden] (q rotated), caches [heads][max_pos][128], these three 16-byte aligned.
 int attn_prefill_tc_launch(const void* qkv, const void* kc, const void* vc, int heads, int hidden, long long max_pos, int pos0, int rows,
-                           void* ctx, cudaStream_t st) {
+                           void* ctx, int* err, bool poll_once, cudaStream_t st) {
     CUtensorMap tm_q, tm_k, tm_v;
     const uint64_t qd[2] = {(uint64_t)hidden, (uint64_t)rows}, qs[1] = {(uint64_t)hidden * 6};
     const uint32_t qb[2] = {64, AT_ROWS};
@@ -364,14 +388,33 @@ int attn_prefill_tc_launch(const void* qkv, const void* kc, const void* vc, int 
     static std::once_flag attr_once[64];
     int dev = 0;
     QW3_CUDA(cudaGetDevice(&dev));
-    auto set_attr = [] { cudaFuncSetAttribute(attn_prefill_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AT_SMEM); };
+    auto set_attr = [] {
+        cudaFuncSetAttribute(attn_prefill_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AT_SMEM);
+        cudaFuncSetAttribute(attn_prefill_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AT_SMEM);
+    };
     if (dev >= 0 && dev < 64) std::call_once(attr_once[dev], set_attr);
     else set_attr();
     AttnParams p = {static_cast<const __half*>(qkv), static_cast<const __half*>(kc), static_cast<const __half*>(vc), max_pos,
-                    static_cast<__half*>(ctx), hidden, pos0, rows};
-    attn_prefill_tc_kernel<<<dim3(heads, (rows + 2 * AT_ROWS - 1) / (2 * AT_ROWS)), AT_THREADS, AT_SMEM, st>>>(tm_q, tm_k, tm_v, p);
+                    static_cast<__half*>(ctx), hidden, pos0, rows, err};
+    const dim3 grid(heads, (rows + 2 * AT_ROWS - 1) / (2 * AT_ROWS));
+    if (poll_once) attn_prefill_tc_kernel<true><<<grid, AT_THREADS, AT_SMEM, st>>>(tm_q, tm_k, tm_v, p);
+    else attn_prefill_tc_kernel<false><<<grid, AT_THREADS, AT_SMEM, st>>>(tm_q, tm_k, tm_v, p);
     QW3_CUDA(cudaGetLastError());
     return QW3_OK;
 }
 
 }  // namespace qw3
+
+extern "C" int qw3_attn_prefill_status(void* stream) {
+    const cudaStream_t st = static_cast<cudaStream_t>(stream);
+    void* word = nullptr;
+    int err = 0;
+    QW3_CUDA(cudaGetSymbolAddress(&word, qw3::g_attn_err));
+    QW3_CUDA(cudaMemcpyAsync(&err, word, 4, cudaMemcpyDeviceToHost, st));
+    QW3_CUDA(cudaStreamSynchronize(st));
+    if (err == 0) return QW3_OK;
+    QW3_CUDA(cudaMemsetAsync(word, 0, 4, st));
+    QW3_CUDA(cudaStreamSynchronize(st));
+    qw3::set_last_error("a bounded device-side wait of qw3_attn_prefill gave up (device error word = 0x%x)", err);
+    return QW3_ERR_TIMEOUT;
+}

@@ -33,7 +33,7 @@ int rmsnorm_rows_launch(const void* x, const void* gamma, int n, float eps, int 
 int rope_kv_rows_launch(void* qkv, void* kc, void* vc, const void* cos_t, const void* sin_t, int hidden, long long max_pos,
                         int pos0, int rows, cudaStream_t st);
 int attn_prefill_launch(const void* qkv, const void* kc, const void* vc, int heads, int hidden, long long max_pos, int pos0,
-                        int rows, void* ctx, cudaStream_t st);
+                        int rows, void* ctx, int* err, cudaStream_t st);
 int gemm_launch(qw3_w4_t w, const void* d_x, int64_t rows, void* d_y, qw3_ws_t ws, void* stream, int epilogue);
 int step_tail_launch(int* d_pos, int* d_step, const int* d_token, int* d_out_ids, int* d_skip, int* d_epoch, bool pdl,
                      cudaStream_t st);
@@ -493,7 +493,7 @@ static int prefill_stage_block(qw3_engine* e, Stage& s, int t0, int rows) {
         QW3_TRY(rmsnorm_rows_launch(s.pf_h, L.gamma, H, c.eps, rows, s.pf_n, s.stream));
         QW3_TRY(qw3_gemm_w4a16(L.wqkv.desc, s.pf_n, rows, s.pf_qkv, s.ws, s.stream));
         QW3_TRY(rope_kv_rows_launch(s.pf_qkv, L.kc, L.vc, s.cos_t, s.sin_t, H, c.max_pos, t0, rows, s.stream));
-        QW3_TRY(attn_prefill_launch(s.pf_qkv, L.kc, L.vc, c.heads, H, c.max_pos, t0, rows, s.pf_ctx, s.stream));
+        QW3_TRY(attn_prefill_launch(s.pf_qkv, L.kc, L.vc, c.heads, H, c.max_pos, t0, rows, s.pf_ctx, ws_struct(s.ws)->err, s.stream));
         QW3_TRY(gemm_launch(L.wo.desc, s.pf_ctx, rows, s.pf_h, s.ws, s.stream, QW3_EPI_RESIDUAL));
         QW3_TRY(rmsnorm_rows_launch(s.pf_h, L.gamma, H, c.eps, rows, s.pf_n, s.stream));
         QW3_TRY(gemm_launch(L.w1.desc, s.pf_n, rows, s.pf_mlp, s.ws, s.stream, QW3_EPI_GELU));

@@ -167,7 +167,7 @@ attn_prefill_kernel(const __half* __restrict__ qkv, const __half* __restrict__ k
 // tensor-core contraction that produces their operand.
 
 int attn_prefill_tc_launch(const void* qkv, const void* kc, const void* vc, int heads, int hidden, long long max_pos, int pos0, int rows,
-                           void* ctx, cudaStream_t st);
+                           void* ctx, int* err, bool poll_once, cudaStream_t st);
 
 // ---- launchers used by the engine (all dimensions even; hidden a multiple of 128) --------------------
 int embed_rows_launch(const void* packed, const void* scale, const void* zp, long long n_alloc, int hidden, long long vocab,
@@ -193,10 +193,10 @@ int rope_kv_rows_launch(void* qkv, void* kc, void* vc, const void* cos_t, const 
     return QW3_OK;
 }
 int attn_prefill_launch(const void* qkv, const void* kc, const void* vc, int heads, int hidden, long long max_pos, int pos0,
-                        int rows, void* ctx, cudaStream_t st) {
+                        int rows, void* ctx, int* err, cudaStream_t st) {
     // A few rows: one CTA per row and head.  From 16 on: the tensor-core kernel, no slower at any length and faster from the first
     // rows on where the cache is long (96 rows at position 2048, 32 heads: 115 us with warp-level MMAs on 64-row tiles, 50 now).
-    if (rows >= 16) return attn_prefill_tc_launch(qkv, kc, vc, heads, hidden, max_pos, pos0, rows, ctx, st);
+    if (rows >= 16) return attn_prefill_tc_launch(qkv, kc, vc, heads, hidden, max_pos, pos0, rows, ctx, err, false, st);
     attn_prefill_kernel<<<dim3(heads, rows), PF_THREADS, 0, st>>>(static_cast<const __half*>(qkv), static_cast<const __half*>(kc),
                                                                   static_cast<const __half*>(vc), hidden, max_pos, pos0,
                                                                   static_cast<__half*>(ctx));
@@ -206,11 +206,26 @@ int attn_prefill_launch(const void* qkv, const void* kc, const void* vc, int hea
 
 }  // namespace qw3
 
-extern "C" int qw3_attn_prefill(const void* d_qkv, const void* d_k_cache, const void* d_v_cache, int32_t heads, int32_t head_dim,
-                                int64_t max_pos, int32_t pos0, int32_t rows, void* d_ctx, void* stream) {
+static int attn_prefill_check(const void* d_qkv, const void* d_k_cache, const void* d_v_cache, int32_t heads, int32_t head_dim,
+                              int64_t max_pos, int32_t pos0, int32_t rows, const void* d_ctx) {
     QW3_REQUIRE(d_qkv && d_k_cache && d_v_cache && d_ctx, "qw3_attn_prefill: null pointer");
     QW3_REQUIRE(head_dim == 128 && heads > 0, "qw3_attn_prefill: head_dim must be 128, heads positive");
     QW3_REQUIRE(rows > 0 && pos0 >= 0 && (int64_t)pos0 + rows <= max_pos, "qw3_attn_prefill: rows out of range");
-    return qw3::attn_prefill_launch(d_qkv, d_k_cache, d_v_cache, heads, heads * 128, max_pos, pos0, rows, d_ctx,
+    return QW3_OK;
+}
+
+extern "C" int qw3_attn_prefill(const void* d_qkv, const void* d_k_cache, const void* d_v_cache, int32_t heads, int32_t head_dim,
+                                int64_t max_pos, int32_t pos0, int32_t rows, void* d_ctx, void* stream) {
+    const int rc = attn_prefill_check(d_qkv, d_k_cache, d_v_cache, heads, head_dim, max_pos, pos0, rows, d_ctx);
+    if (rc != QW3_OK) return rc;
+    return qw3::attn_prefill_launch(d_qkv, d_k_cache, d_v_cache, heads, heads * 128, max_pos, pos0, rows, d_ctx, nullptr,
                                     static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int qw3_attn_prefill_poll_once(const void* d_qkv, const void* d_k_cache, const void* d_v_cache, int32_t heads, int32_t head_dim,
+                                          int64_t max_pos, int32_t pos0, int32_t rows, void* d_ctx, void* stream) {
+    const int rc = attn_prefill_check(d_qkv, d_k_cache, d_v_cache, heads, head_dim, max_pos, pos0, rows, d_ctx);
+    if (rc != QW3_OK) return rc;
+    return qw3::attn_prefill_tc_launch(d_qkv, d_k_cache, d_v_cache, heads, heads * 128, max_pos, pos0, rows, d_ctx, nullptr, true,
+                                       static_cast<cudaStream_t>(stream));
 }

@@ -161,6 +161,15 @@ int qw3_attn_decode(const void* d_q, const void* d_k_cache, const void* d_v_cach
  * of 64 cache rows), below that one CTA per row. */
 int qw3_attn_prefill(const void* d_qkv, const void* d_k_cache, const void* d_v_cache, int32_t heads, int32_t head_dim,
                      int64_t max_pos, int32_t pos0, int32_t rows, void* d_ctx, void* stream);
+/* Companion of qw3_attn_prefill, which takes no workspace (as qw3_gemv_w4a16_noalloc_status is of the GEMV without one): a wait that
+ * gives up inside the kernel writes NaN rows and a code into an error word of the library on that GPU.  Reads and clears the word of
+ * the current device: QW3_ERR_TIMEOUT if a call since the last check gave up, QW3_OK otherwise.  Synchronises `stream`.  The
+ * engine's prompt phase records into its own workspace and returns QW3_ERR_TIMEOUT by itself. */
+int qw3_attn_prefill_status(void* stream);
+/* Test hook for that path (as qw3_handoff_wait is for the hand-off): the tensor-core kernel at any number of rows, with waits that look
+ * at their barrier once and give up.  Every row of d_ctx comes back as a result or as NaN. */
+int qw3_attn_prefill_poll_once(const void* d_qkv, const void* d_k_cache, const void* d_v_cache, int32_t heads, int32_t head_dim,
+                               int64_t max_pos, int32_t pos0, int32_t rows, void* d_ctx, void* stream);
 
 /* Embedding column gather straight from the packed [hidden][vocab] matrix (gather lambda,
  * Inference.cu:1310-1315).  Token from *d_token when it is not NULL, else `token`. */

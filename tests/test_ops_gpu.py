@@ -131,6 +131,27 @@ def test_attention_prefill_nothing_behind_a_row_reaches_it(ops, orc, cuda, heads
         assert (_ulp_diff(got[r][ok], want[ok]) > 1).sum() <= 0.01 * ok.sum(), r
 
 
+def test_attention_prefill_reports_a_wait_that_gives_up(ops, orc, cuda):
+    """Waits that look at their barrier once: the softmax warps do so long before the first copy has landed.  The kernel returns,
+    the status call reports it once, no row holds anything but its result or NaN, and the next call is right."""
+    cabi = ops.cabi
+    heads, max_pos, pos0, rows = 2, 700, 100, 300
+    H = heads * 128
+    qkv, kc, vc = (orc.gen_normal_f16(35, kind, n) for kind, n in ((orc.ACT, rows * 3 * H), (orc.KV_K, H * max_pos), (orc.KV_V, H * max_pos)))
+    dq, dk, dv = _to_dev(qkv.reshape(rows, 3 * H), cuda), _to_dev(kc, cuda), _to_dev(vc, cuda)
+    L, st = cabi.lib(), ops._stream()
+    want = ops.attn_prefill(dq, dk, dv, heads, max_pos, pos0, rows)
+    cabi.check(L.qw3_attn_prefill_status(st), "qw3_attn_prefill_status")
+    got = torch.zeros_like(want)
+    cabi.check(L.qw3_attn_prefill_poll_once(dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), heads, 128, max_pos, pos0, rows, got.data_ptr(), st),
+               "qw3_attn_prefill_poll_once")
+    assert L.qw3_attn_prefill_status(st) == cabi.QW3_ERR_TIMEOUT and b"0x3002" in L.qw3_last_error()
+    assert L.qw3_attn_prefill_status(st) == cabi.QW3_OK
+    assert (torch.isnan(got) | (got == want)).all() and torch.isnan(got).any()
+    assert torch.equal(ops.attn_prefill(dq, dk, dv, heads, max_pos, pos0, rows), want)
+    cabi.check(L.qw3_attn_prefill_status(st), "qw3_attn_prefill_status")
+
+
 def test_embed_gather_bit_exact(ops, orc, cuda):
     H, V = 512, 4096 + 256
     p, s, z = orc.gen_linear(24, H, V, kind=orc.EMB)
