@@ -80,9 +80,9 @@ gemm_w4a16_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const GemmParam
     uint64_t* bars = reinterpret_cast<uint64_t*>(x_st + GM_X_STAGES * x_bytes);
     const uint32_t a_full = smem_u32(bars + 2 * GM_MAX_STAGES), a_empty = smem_u32(bars + 3 * GM_MAX_STAGES);
     const uint32_t x_full = smem_u32(bars + 4 * GM_MAX_STAGES), x_empty = a_empty;   // one release barrier per stage
-    const uint32_t acc_full = smem_u32(bars + 6 * GM_MAX_STAGES);
+    const uint32_t acc_full = smem_u32(bars + 6 * GM_MAX_STAGES), drain = smem_u32(bars);   // drain: one an issuer
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 6 * GM_MAX_STAGES + 1);
-    int* s_dead = reinterpret_cast<int*>(tmem_slot + 1);   // bars: (6 * 24 + 2) * 8 bytes < 1280
+    volatile int* s_dead = reinterpret_cast<volatile int*>(tmem_slot + 1);   // bars: (6 * 24 + 2) * 8 bytes < 1280
 
     const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
     const int tile_m = blockIdx.x, tile_n = blockIdx.y;
@@ -100,6 +100,8 @@ gemm_w4a16_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const GemmParam
             mbar_init(a_empty + 8 * s, 1);      // commit of the MMAs that read A and X of the stage
         }
         mbar_init(acc_full, 2);             // the last commit of each of the two MMA issuers
+        mbar_init(drain, 1);
+        mbar_init(drain + 8, 1);
         *s_dead = 0;
         mbar_fence_init();
     }
@@ -119,16 +121,20 @@ gemm_w4a16_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const GemmParam
         if (elect_one()) {
             tma_prefetch_desc(&tmap_x);
             bool ok = true;
+            int issued = 0;
             for (int kb = 0; kb < n_kb && ok; ++kb) {
                 const int s = kb % GM_X_STAGES;
                 if (kb >= GM_X_STAGES) ok = mbar_wait(x_empty + 8 * s, ((kb / GM_X_STAGES) - 1) & 1);   // freed by the MMAs' commit
                 if (!ok) break;
                 mbar_expect_tx(x_full + 8 * s, (uint32_t)x_bytes);
                 tma_load_2d(smem_u32(x_st + s * x_bytes), &tmap_x, (kb_lo + kb) * GM_BK, tile_n * p.n_tile, x_full + 8 * s);
+                ++issued;
             }
             if (!ok) {
                 atomicCAS(p.err, 0, 0x30001);
                 *s_dead = 1;
+                for (int kb = issued > GM_X_STAGES ? issued - GM_X_STAGES : 0; kb < issued; ++kb)   // the copies in flight
+                    mbar_wait(x_full + 8 * (kb % GM_X_STAGES), (uint32_t)(kb / GM_X_STAGES) & 1u);
             }
         }
     } else if (warp == 1 || warp == GM_ISSUER_B) {
@@ -181,6 +187,10 @@ gemm_w4a16_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const GemmParam
                     atomicCAS(p.err, 0, 0x30006);
                     *s_dead = 1;
                 }
+            }
+            if (*s_dead != 0) {   // some wait gave up: the MMAs in flight
+                umma_commit(drain + 8 * who);
+                mbar_wait(drain + 8 * who, 0);
             }
         }
         __syncwarp();
@@ -410,6 +420,24 @@ __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
     return r;
 }
 
+// A wait of the leader's MMA issuer has given up: it waits for the copies of the activations in flight.  Both producers give up after it
+// at the latest (no commit frees their stages) and then leave 1 + the K blocks they have asked for in `asked`, the peer from its own
+// SM.  A lap of a stage completes with the leader's expectation and the bytes of both CTAs; they are never more than a lap apart.
+__device__ __noinline__ void pair_drain(uint32_t x_full, const volatile int* asked, uint32_t half_bytes) {
+    const long long t0 = clock64();
+    while (asked[0] == 0 || asked[1] == 0)
+        if (clock64() - t0 > (1ll << 32)) return;
+    for (int s = 0; s < GP_STAGES; ++s) {
+        const int laps0 = (asked[0] - 1 - s + GP_STAGES - 1) / GP_STAGES, laps1 = (asked[1] - 1 - s + GP_STAGES - 1) / GP_STAGES;
+        const int laps = max(laps0, laps1);
+        if (laps <= 0) continue;
+        if (laps1 > laps0) mbar_expect_tx(x_full + 8 * s, half_bytes);   // the peer's half alone is on its way
+        else if (laps0 > laps1)                                          // the peer's half will not come
+            asm volatile("mbarrier.complete_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(x_full + 8 * s), "r"(half_bytes) : "memory");
+        mbar_wait(x_full + 8 * s, (uint32_t)(laps - 1) & 1u);
+    }
+}
+
 // One work item: tile and K range.  Neighbouring items share the 256 outputs and differ in the rows.
 struct PairItem { int tile_m, tile_n, kb_lo, n_kb, slot; };   // slot: place of the partial products, negative: none
 __device__ __forceinline__ PairItem pair_item(const PairParams& p, int item) {
@@ -456,6 +484,8 @@ gemm_w4a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const PairPar
     const uint32_t pk_full = smem_u32(bars + 3 * GP_STAGES + 2), pk_empty = pk_full + 8 * GP_PK_STAGES;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 3 * GP_STAGES + 2 + 2 * GP_PK_STAGES);
     volatile int* s_dead = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    volatile int* s_asked = s_dead + 1;   // pair_drain
+    const uint32_t drain = smem_u32(tmem_slot + 4);
 
     const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
     const int rank = (int)cluster_rank();
@@ -473,7 +503,8 @@ gemm_w4a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const PairPar
         }
         mbar_init(acc_full, 1);                 // commit of an item's last MMAs
         mbar_init(acc_empty, 2 * GP_WARPS);     // every epilogue warp of the pair has read its share
-        *s_dead = 0;
+        mbar_init(drain, 1);
+        *s_dead = s_asked[0] = s_asked[1] = 0;
         mbar_fence_init();
     }
     for (int g = tid; g < p.Kb; g += GP_THREADS) tab[g] = pack_h2(p.zp[g % p.n_alloc], p.scale[g % p.n_alloc]);
@@ -491,7 +522,7 @@ gemm_w4a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const PairPar
         if (elect_one()) {
             tma_prefetch_desc(&tmap_x);
             const int half_n = p.n_tile / 2;
-            int s = 0;
+            int s = 0, asked = 0;
             uint32_t phase = 0;
             bool ok = true, wrapped = false;
             for (int item = first; item < items && ok; item += step) {
@@ -502,6 +533,7 @@ gemm_w4a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const PairPar
                     if (rank == 0) mbar_expect_tx(x_full + 8 * s, (uint32_t)p.n_tile * 128u);
                     tma_load_2d_pair(smem_u32(x_st + s * GP_X_BYTES), &tmap_x, (w.kb_lo + kb) * GM_BK,
                                      w.tile_n * p.n_tile + rank * half_n, x_full + 8 * s);
+                    ++asked;
                     if (++s == GP_STAGES) { s = 0; phase ^= 1u; wrapped = true; }
                 }
             }
@@ -511,6 +543,12 @@ gemm_w4a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const PairPar
             if (!ok) {
                 atomicCAS(p.err, 0, 0x30011);
                 *s_dead = 1;
+                const uint32_t word = smem_u32(const_cast<int*>(s_asked)) + 4 * rank;   // in the leader
+                asm volatile(
+                    "{\n\t.reg .b32 a;\n\t"
+                    "mapa.shared::cluster.u32 a, %0, 0;\n\t"
+                    "st.shared::cluster.u32 [a], %1;\n\t}"
+                    ::"r"(word), "r"(asked + 1) : "memory");
             }
         }
         __syncwarp();
@@ -546,6 +584,9 @@ gemm_w4a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const PairPar
             if (!ok) {
                 atomicCAS(p.err, 0, 0x30012);
                 *s_dead = 1;
+                asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(drain) : "memory");
+                mbar_wait(drain, 0);   // the MMAs in flight
+                pair_drain(x_full, s_asked, (uint32_t)p.n_tile * 64u);
             }
         }
         __syncwarp();
