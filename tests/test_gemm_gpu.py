@@ -103,3 +103,20 @@ def test_gemm_pairs_edges(ops, orc, cuda, M, K, R, integral):
     d = _ulp_diff(y.cpu().numpy(), got)
     near = np.abs(y.cpu().numpy().astype(np.float32) - got.astype(np.float32)) <= 1e-4 * np.abs(y32).mean()
     assert ((d <= 1) | near).all() and (d > 0).mean() < 0.08
+
+
+@pytest.mark.parametrize("M,K,R", [(12288, 4096, 2048), (4096, 12288, 300)])
+def test_gemm_pairs_repeat_bitwise(ops, orc, cuda, M, K, R):
+    """Several waves of tiles, and single tiles with long sums, 60 launches each: an operand that one CTA of a pair reads before the
+    other's writes have arrived would show as a difference between launches."""
+    p, s, z = orc.gen_linear(46, M, K)
+    ws = ops.Workspace()
+    w = ops.W4Linear(_to_dev(p, cuda), _to_dev(s, cuda), _to_dev(z, cuda), M, K)
+    x = _to_dev(orc.gen_normal_f16(46, orc.ACT, R * K).reshape(R, K), cuda)
+    first = torch.zeros(R, M, dtype=torch.float16, device=cuda)
+    ops.gemm_w4a16(w, ws, x, first)
+    y = torch.zeros_like(first)
+    for _ in range(60):
+        ops.gemm_w4a16(w, ws, x, y)
+        assert torch.equal(y, first)
+    ws.check()
