@@ -336,7 +336,7 @@ __global__ void gemm_splitk_reduce_kernel(const float* __restrict__ part, int sp
 // own 128 outputs and holds half of the activation rows, so that a K block moves half the operand-B bytes through an SM's
 // shared memory (A 16 KB written + 16 KB read, B 16 KB + 16 KB, in the 512 cycles the MMAs take at 256 rows) and half through L2.
 //   warp 0      TMA producer of this CTA's half of the activation rows
-//   warp 1      MMA issuer (leader CTA of the pair only), even / odd K blocks into two accumulators
+//   warp 1      MMA issuer (leader CTA of the pair only), K blocks in turn into two to four accumulators
 //   warps 2..17 unpack (four groups of four warps take the K blocks in turn), epilogue
 //   warp 18     loader: the packed bytes of this CTA's outputs into a ring of twelve K blocks (cp.async, 64 bytes of a row; a tensor
 //               copy of such a narrow box costs more than all else in the CTA).  The unpack warps must not have loads
@@ -364,6 +364,7 @@ struct PairParams {
     const __half* zp;
     int n_alloc, M, K, Mb, Kb;
     int rows, n_tile, n_tiles_n, n_tiles_m;
+    int n_acc, acc_stride;   // accumulators of a tile, which its K blocks take in turn, and the columns between them
     int full;          // tiles whose K is not split
     int splits;        // parts of the K of each of the tiles after those
     int items;         // full + splits * (the other tiles)
@@ -511,7 +512,7 @@ gemm_w4a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const PairPar
         mbar_fence_init();
     }
     for (int g = tid; g < p.Kb; g += GP_THREADS) tab[g] = pack_h2(p.zp[g % p.n_alloc], p.scale[g % p.n_alloc]);
-    if (warp == 1) {   // all 512 columns: two accumulators of up to 256
+    if (warp == 1) {   // all 512 columns
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
@@ -567,6 +568,7 @@ gemm_w4a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const PairPar
                 const PairItem w = pair_item(p, item);
                 if (n > 0 && !(ok = mbar_wait(acc_empty, (uint32_t)(n - 1) & 1u))) break;
                 tc_fence_after();
+                int acc = 0;
                 for (int kb = 0; kb < w.n_kb; ++kb) {
                     if (*s_dead != 0 || !mbar_wait(x_full + 8 * s, phase) || !mbar_wait(a_full + 8 * s, phase)) {
                         ok = false;
@@ -575,11 +577,12 @@ gemm_w4a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const PairPar
                     tc_fence_after();
                     const uint64_t adesc = adesc0 + (uint64_t)(uint32_t)(s * (GM_A_BYTES >> 4));
                     const uint64_t bdesc = bdesc0 + (uint64_t)(uint32_t)(s * (GP_X_BYTES >> 4));
-                    const uint32_t d = tmem_base + (uint32_t)((kb & 1) * GP_MAX_N);
+                    const uint32_t d = tmem_base + (uint32_t)(acc * p.acc_stride);
 #pragma unroll
                     for (int ks = 0; ks < GM_BK / 16; ++ks)
-                        umma_f16_pair(d, adesc + (uint64_t)(2 * ks), bdesc + (uint64_t)(2 * ks), idesc, (kb >= 2 || ks > 0) ? 1u : 0u);
+                        umma_f16_pair(d, adesc + (uint64_t)(2 * ks), bdesc + (uint64_t)(2 * ks), idesc, (kb >= p.n_acc || ks > 0) ? 1u : 0u);
                     umma_commit_pair(st_empty + 8 * s);
+                    if (++acc == p.n_acc) acc = 0;
                     if (++s == GP_STAGES) { s = 0; phase ^= 1u; }
                 }
                 if (ok) umma_commit_pair(acc_full);
@@ -723,9 +726,14 @@ gemm_w4a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const PairPar
                 tmem_ld16(tmem_base + ((uint32_t)(32 * q) << 16) + (uint32_t)c0, v);
 #pragma unroll
                 for (int e = 0; e < 16; ++e) f[e] = __uint_as_float(v[e]);
-                tmem_ld16(tmem_base + ((uint32_t)(32 * q) << 16) + (uint32_t)(GP_MAX_N + c0), v);
+                tmem_ld16(tmem_base + ((uint32_t)(32 * q) << 16) + (uint32_t)(p.acc_stride + c0), v);
 #pragma unroll
                 for (int e = 0; e < 16; ++e) f[e] += __uint_as_float(v[e]);
+                for (int acc = 2; acc < p.n_acc; ++acc) {   // in a fixed order
+                    tmem_ld16(tmem_base + ((uint32_t)(32 * q) << 16) + (uint32_t)(acc * p.acc_stride + c0), v);
+#pragma unroll
+                    for (int e = 0; e < 16; ++e) f[e] += __uint_as_float(v[e]);
+                }
                 if (!valid) continue;
                 if (w.slot >= 0) {
                     float* dst = p.part + ((size_t)w.slot * p.n_tile + c0) * 256 + rank * 128 + m;
@@ -831,27 +839,57 @@ static int encode_rows(CUtensorMap* map, const void* x, int64_t rows, int64_t K,
     return encode_f16_map(map, x, 2, dims, strides, box);
 }
 
+// How the one-CTA kernel cuts rows x M x K: few rows and few output tiles leave most SMs without a CTA, so K is split over grid.z (fp32
+// partial products in the workspace, summed in split order by a second kernel) until ~one CTA per SM, while the partials fit.
+struct OneCut { int n_tile, n_acc, ctas, splits; };
+static OneCut one_cut(long long rows, long long M, int K, int sm_count) {
+    OneCut c;
+    c.n_tile = rows <= 16 ? 16 : rows <= 32 ? 32 : rows <= 64 ? 64 : rows <= 128 ? 128 : 256;
+    c.n_acc = c.n_tile <= 64 ? 4 : 2;       // half of them per MMA issuer
+    const long long ctas = (M / GM_TILE_M) * ((rows + c.n_tile - 1) / c.n_tile);
+    c.ctas = (int)ctas;
+    c.splits = 1;
+    while (c.splits < 8 && ctas * (c.splits * 2) <= sm_count && (K / GM_BK) / (c.splits * 2) >= 8 &&
+           (long long)(c.splits * 2) * rows * M <= (long long)WS_PARTIALS)
+        c.splits *= 2;
+    return c;
+}
+// MMAs that one accumulator of it sums (an issuer has every other K block, and two accumulators where there are four).  The error grows
+// with that (64 rows of 151936 x 4096: 0.53 % of the results are not the nearest fp16 at 64 MMAs, 0.95 % at 128), so the pair kernel
+// takes no cut in which it is more.
+static int one_sum(const OneCut& c, int K) { return ((K / GM_BK + c.splits - 1) / c.splits + 1) / 2 * (2 * GM_BK / 16) / c.n_acc; }
+// Accumulators (fewest: each is one more pass of the epilogue over tensor memory) with which n_kb blocks give sums of at most `longest`
+// MMAs; 0: more than 512 columns hold.
+static int pair_accumulators(int n_kb, int n_tile, int longest) {
+    for (int a = 2; a <= 4 && a * n_tile <= 512; ++a)
+        if ((n_kb + a - 1) / a * (GM_BK / 16) <= longest) return a;
+    return 0;
+}
+
 // How rows x M x K is cut for the pair kernel: the width of a row tile and the K splits of the tiles that do not fill a wave of
 // pairs.  The estimate counts K blocks: an MMA step of n_tile rows takes 2 n_tile cycles, and a K block is never cheaper than
 // its unpacking; a split tile pays for its partial products and the second kernel.
-struct PairCut { int n_tile, full, splits, items; };
-static PairCut pair_cut(long long rows, int M, int K, int pairs) {
+struct PairCut { int n_tile, n_acc, full, splits, items; };
+static PairCut pair_cut(long long rows, int M, int K, int pairs, int longest) {   // n_tile 0: no cut with sums of at most `longest`
     const int n_kb = K / GM_BK, tiles_m = (M + 255) / 256;
     PairCut best = {};
     double best_cost = 0.0;
     for (int n = 32; n <= GP_MAX_N; n += 32) {
-        if (n < GP_MAX_N && n * 2 <= rows && n < 160) continue;   // narrow tiles only where few of them cover the rows
+        if (n < GP_MAX_N && n * 2 <= rows && n < 96) continue;   // narrow tiles only where few of them cover the rows
         const long long tiles = tiles_m * ((rows + n - 1) / n);
         const double kb_cost = n > 128 ? 2.0 * n : 256.0;
         const int tail = (int)(tiles % pairs);
         const long long waves = tiles / pairs;
         for (int z = 1; z <= 16 && n_kb / z >= 8; ++z) {
             if (z > 1 && (tail == 0 || (long long)tail * z * n > (long long)(WS_PARTIALS / 256))) break;
+            const int n_acc = pair_accumulators(z > 1 && tiles == tail ? (n_kb + z - 1) / z : n_kb, n, longest);
+            if (n_acc == 0) continue;
             const int tail_waves = (tail * z + pairs - 1) / pairs;
             const double cost = waves * (n_kb * kb_cost + 2000.0) + tail_waves * ((n_kb + z - 1) / z * kb_cost + 2000.0) + (z > 1 ? 6000.0 : 0.0);
             if (best.n_tile == 0 || cost < best_cost) {
                 best_cost = cost;
                 best.n_tile = n;
+                best.n_acc = n_acc;
                 best.full = (int)(z > 1 ? tiles - tail : tiles);
                 best.splits = z;
                 best.items = best.full + (z > 1 ? tail * z : 0);
@@ -869,8 +907,9 @@ static PairCut pair_cut(long long rows, int M, int K, int pairs) {
 static bool pair_wanted(const W4Desc* d, long long rows, const void* d_y, const Workspace* ws) {
     const int pairs = ws->sm_count / 2;
     if (d->K / GM_BK < 2 * GP_GROUPS || pairs < 1 || (reinterpret_cast<uintptr_t>(d_y) & 15) != 0) return false;
+    const PairCut cut = pair_cut(rows, (int)d->M, (int)d->K, pairs, one_sum(one_cut(rows, d->M, (int)d->K, ws->sm_count), (int)d->K));
+    if (cut.n_tile == 0) return false;
     if (rows <= 128) return (d->M + 255) / 256 >= pairs;
-    const PairCut cut = pair_cut(rows, (int)d->M, (int)d->K, pairs);
     return cut.splits > 1 || cut.items <= pairs;
 }
 
@@ -881,7 +920,9 @@ static int pair_launch(const W4Desc* d, const void* d_x, long long rows, void* d
     p.M = (int)d->M; p.K = (int)d->K; p.Mb = p.M / 128; p.Kb = p.K / 128;
     p.rows = (int)rows;
     const int pairs = ws->sm_count / 2;
-    const PairCut cut = pair_cut(rows, p.M, p.K, pairs);
+    const PairCut cut = pair_cut(rows, p.M, p.K, pairs, one_sum(one_cut(rows, p.M, p.K, ws->sm_count), p.K));
+    p.n_acc = cut.n_acc;
+    p.acc_stride = 512 / p.n_acc & ~31;
     p.n_tile = cut.n_tile; p.full = cut.full; p.splits = cut.splits; p.items = cut.items;
     p.n_tiles_m = (p.M + 255) / 256;
     p.n_tiles_n = (int)((rows + p.n_tile - 1) / p.n_tile);
@@ -947,8 +988,9 @@ int qw3::gemm_launch(qw3_w4_t w, const void* d_x, int64_t rows, void* d_y, qw3_w
     p.M = (int)d->M; p.K = (int)d->K; p.Mb = p.M / 128; p.Kb = p.K / 128;
     p.uniform = d->uniform; p.exact = d->zp_integral;
     p.rows = (int)rows;
-    p.n_tile = rows <= 16 ? 16 : rows <= 32 ? 32 : rows <= 64 ? 64 : rows <= 128 ? 128 : 256;
-    p.n_acc = p.n_tile <= 64 ? 4 : 2;       // half of them per MMA issuer
+    const OneCut cut = one_cut(rows, d->M, p.K, ws_struct(ws)->sm_count);
+    p.n_tile = cut.n_tile;
+    p.n_acc = cut.n_acc;
     p.acc_stride = p.n_tile < 32 ? 32 : p.n_tile;
     p.tmem_cols = p.n_acc * p.acc_stride;   // 128, 128, 256, 256, 512 columns: powers of two
     p.y = static_cast<__half*>(d_y);
@@ -970,14 +1012,7 @@ int qw3::gemm_launch(qw3_w4_t w, const void* d_x, int64_t rows, void* d_y, qw3_w
             cudaFuncSetAttribute(gemm_w4a16_tc_kernel<6>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
             cudaFuncSetAttribute(gemm_w4a16_tc_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
         });
-    // Few rows and few output tiles leave most SMs without a CTA: split K over grid.z (fp32 partial products in the
-    // workspace, summed in split order by a second kernel) until ~one CTA per SM, while the partials fit.
-    const long long ctas = (d->M / GM_TILE_M) * ((rows + p.n_tile - 1) / p.n_tile);
-    const long long part_cap = (long long)WS_PARTIALS;   // floats in the workspace
-    int splits = 1;
-    while (splits < 8 && ctas * (splits * 2) <= ws_struct(ws)->sm_count && (p.K / GM_BK) / (splits * 2) >= 8 &&
-           (long long)(splits * 2) * rows * d->M <= part_cap)
-        splits *= 2;
+    const int splits = cut.splits;
     p.part = splits > 1 ? ws_struct(ws)->partials : nullptr;
     dim3 grid((unsigned)(d->M / GM_TILE_M), (unsigned)((rows + p.n_tile - 1) / p.n_tile), (unsigned)splits);
     const cudaStream_t st = static_cast<cudaStream_t>(stream);

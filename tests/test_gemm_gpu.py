@@ -120,3 +120,21 @@ def test_gemm_pairs_repeat_bitwise(ops, orc, cuda, M, K, R):
         ops.gemm_w4a16(w, ws, x, y)
         assert torch.equal(y, first)
     ws.check()
+
+
+@pytest.mark.parametrize("M,K,R", [(19200, 4096, 64), (4096, 1024, 256)])
+def test_gemm_pairs_sum_no_longer_than_one_cta(ops, orc, cuda, M, K, R):
+    """The error of a result grows with the number of MMAs that one accumulator sums.  Share of results that are not the nearest fp16 of
+    the 64-bit sum: the pairs' against the one-CTA kernel's (a result off 16 bytes), of some hundred each, so that twice the
+    length (1.8 times the share) is ten standard deviations away from the bound."""
+    p, s, z = orc.gen_linear(47, M, K)
+    X = orc.gen_normal_f16(47, orc.ACT, R * K).reshape(R, K)
+    rows = np.arange(0, R, R // 64 * 4 if M < 10000 else R // 16)
+    _, want = orc.gemm_w4a16(p, s, z, M, K, X[rows])
+    got, w, ws = _gemm(ops, cuda, p, s, z, M, K, X)
+    off = torch.zeros(R * M + 8, dtype=torch.float16, device=cuda)
+    ops.gemm_w4a16(w, ws, _to_dev(X, cuda), off[2:2 + R * M].view(R, M))
+    ws.check()
+    one = off[2:2 + R * M].view(R, M).cpu().numpy()
+    pairs, ref = (got[rows] != want).sum(), (one[rows] != want).sum()
+    assert ref > 100 and pairs <= 1.3 * ref
