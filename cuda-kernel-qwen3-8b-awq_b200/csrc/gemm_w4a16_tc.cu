@@ -867,60 +867,71 @@ static int pair_accumulators(int n_kb, int n_tile, int longest) {
 }
 
 // How rows x M x K is cut for the pair kernel: the width of a row tile and the K splits of the tiles that do not fill a wave of
-// pairs.  The estimate counts K blocks: an MMA step of n_tile rows takes 2 n_tile cycles, and a K block is never cheaper than
-// its unpacking; a split tile pays for its partial products and the second kernel.
-struct PairCut { int n_tile, n_acc, full, splits, items; };
+// pairs; the cut with the lowest estimate, in us.  A K block takes 0.33 us at up to 128 rows (whatever the rows: the hand-over) and 0.39 at
+// 256; an item 2.3 (epilogue) and 0.3 for each further pass over 128 rows of accumulators; the sum of split tiles 4 and 0.7 for a
+// million partial products; a call 5.  Over 520 sizes the cut taken is 0.6 % slower than the fastest of those tried in the mean, 7 % in
+// the 99th percentile.
+struct PairCut { int n_tile, n_acc, full, splits, items; double us; };
 static PairCut pair_cut(long long rows, int M, int K, int pairs, int longest) {   // n_tile 0: no cut with sums of at most `longest`
     const int n_kb = K / GM_BK, tiles_m = (M + 255) / 256;
+    const int max_z = n_kb / 8 < 16 ? n_kb / 8 : 16;
+    int kbs[17];   // K blocks of a part
+    for (int z = 1; z <= max_z; ++z) kbs[z] = (n_kb + z - 1) / z;
     PairCut best = {};
-    double best_cost = 0.0;
-    for (int n = 32; n <= GP_MAX_N; n += 32) {
-        if (n < GP_MAX_N && n * 2 <= rows && n < 96) continue;   // narrow tiles only where few of them cover the rows
+    for (int n = 32; n <= GP_MAX_N && n - 32 < rows; n += 32) {
         const long long tiles = tiles_m * ((rows + n - 1) / n);
-        const double kb_cost = n > 128 ? 2.0 * n : 256.0;
-        const int tail = (int)(tiles % pairs);
+        const double kb_us = n > 128 ? 0.33 + 0.06 * (n - 128) / 128 : 0.33;
         const long long waves = tiles / pairs;
-        for (int z = 1; z <= 16 && n_kb / z >= 8; ++z) {
-            if (z > 1 && (tail == 0 || (long long)tail * z * n > (long long)(WS_PARTIALS / 256))) break;
-            const int n_acc = pair_accumulators(z > 1 && tiles == tail ? (n_kb + z - 1) / z : n_kb, n, longest);
+        const int tail = (int)(tiles - waves * pairs);
+        for (int z = 1; z <= max_z; ++z) {   // in more than two waves the parts of a tail are no gain
+            if (z > 1 && (tail == 0 || tail * z > 2 * pairs || tail * z * n > (int)(WS_PARTIALS / 256))) break;
+            const int n_acc = pair_accumulators(z > 1 && waves == 0 ? kbs[z] : n_kb, n, longest);
             if (n_acc == 0) continue;
-            const int tail_waves = (tail * z + pairs - 1) / pairs;
-            const double cost = waves * (n_kb * kb_cost + 2000.0) + tail_waves * ((n_kb + z - 1) / z * kb_cost + 2000.0) + (z > 1 ? 6000.0 : 0.0);
-            if (best.n_tile == 0 || cost < best_cost) {
-                best_cost = cost;
+            const int tail_waves = tail == 0 ? 0 : tail * z <= pairs ? 1 : 2;
+            const double item_us = 2.3 + 0.3 * (n_acc - 1) * n / 128;
+            const double us = 5.0 + waves * (n_kb * kb_us + item_us) + tail_waves * (kbs[z] * kb_us + item_us) +
+                              (z > 1 ? 4.0 + 0.7e-6 * 256 * tail * z * n : 0.0);
+            if (best.n_tile == 0 || us < best.us) {
                 best.n_tile = n;
                 best.n_acc = n_acc;
                 best.full = (int)(z > 1 ? tiles - tail : tiles);
                 best.splits = z;
                 best.items = best.full + (z > 1 ? tail * z : 0);
+                best.us = us;
             }
         }
     }
     return best;
 }
 
-// Where the pairs are the faster kernel (us, one-CTA kernel / pairs).  More than 128 rows: 12288 x 4096 34.9 / 26.8 at 160 rows and
-// 202 / 156 at 2048, 4096 x 12288 79.5 / 65.9 at 512 rows; but where neither a single wave nor a split of the last one
-// fills the chip the smaller tiles win (4096 x 12288 at 2048 rows 175 / 208).  Up to 128 rows a call is short and the pairs' start
-// and second kernel show (4096 x 4096 at 64 rows 16.4 / 20.6), unless there are 256-output tiles for every pair of SMs
-// (151936 x 4096 at 64 rows 251 / 190).  The result is stored by 16 bytes; an item has two K blocks for each unpack group.
-static bool pair_wanted(const W4Desc* d, long long rows, const void* d_y, const Workspace* ws) {
-    const int pairs = ws->sm_count / 2;
-    if (d->K / GM_BK < 2 * GP_GROUPS || pairs < 1 || (reinterpret_cast<uintptr_t>(d_y) & 15) != 0) return false;
-    const PairCut cut = pair_cut(rows, (int)d->M, (int)d->K, pairs, one_sum(one_cut(rows, d->M, (int)d->K, ws->sm_count), (int)d->K));
-    if (cut.n_tile == 0) return false;
-    if (rows <= 128) return (d->M + 255) / 256 >= pairs;
-    return cut.splits > 1 || cut.items <= pairs;
+// The pairs where their estimate is the lower one (us, one-CTA kernel / pairs; 12288 x 4096: 35 / 28 at 160 rows, 68 / 53 at 512, 101 / 82 at
+// 1024, 202 / 165 at 2048; 4096 x 12288 175 / 154 at 2048).  The one-CTA kernel stays ahead where it splits K and the workspace
+// does not hold the partial products of as many parts of the pairs' tiles (4096 x 12288 at 280 rows 50 / 64, 8192 x 8192 at 129 rows
+// 52 / 62) and with a single block of outputs, which leaves half of each pair idle (128 x 12288 at 1953 rows 26 / 29).  Up to 128 rows
+// a call is short and the pairs' start and second kernel show (4096 x 4096 at 64 rows 16.4 / 20.6; 18944 x 2048, one wave of both,
+// 20.0 / 20.6), unless there are more 256-output tiles than pairs of SMs (151936 x 4096 at 64 rows 250 / 196).  The result is stored by
+// 16 bytes; an item has two K blocks for each unpack group.
+static bool pair_wanted(const W4Desc* d, long long rows, const void* d_y, const Workspace* ws, PairCut* cut) {
+    const int pairs = ws->sm_count / 2, K = (int)d->K;
+    if (K / GM_BK < 2 * GP_GROUPS || pairs < 1 || (reinterpret_cast<uintptr_t>(d_y) & 15) != 0) return false;
+    if (rows <= 128 && (d->M + 255) / 256 <= pairs) return false;
+    const OneCut one = one_cut(rows, d->M, K, ws->sm_count);
+    *cut = pair_cut(rows, (int)d->M, K, pairs, one_sum(one, K));
+    if (cut->n_tile == 0) return false;
+    if (rows <= 128) return true;
+    const long long waves = (one.ctas * one.splits + ws->sm_count - 1) / ws->sm_count;
+    const double one_us = 2.4 + waves * ((K / GM_BK + one.splits - 1) / one.splits * 0.433 + 10.5) + (one.splits > 1 ? 2.6 : 0.0);
+    return cut->us <= one_us;
 }
 
-static int pair_launch(const W4Desc* d, const void* d_x, long long rows, void* d_y, const Workspace* ws, cudaStream_t st, int epilogue) {
+static int pair_launch(const W4Desc* d, const PairCut& cut, const void* d_x, long long rows, void* d_y, const Workspace* ws, cudaStream_t st,
+                       int epilogue) {
     PairParams p = {};
     p.packed = d->packed;
     p.scale = d->scale; p.zp = d->zp; p.n_alloc = (int)d->n_alloc;
     p.M = (int)d->M; p.K = (int)d->K; p.Mb = p.M / 128; p.Kb = p.K / 128;
     p.rows = (int)rows;
     const int pairs = ws->sm_count / 2;
-    const PairCut cut = pair_cut(rows, p.M, p.K, pairs, one_sum(one_cut(rows, p.M, p.K, ws->sm_count), p.K));
     p.n_acc = cut.n_acc;
     p.acc_stride = 512 / p.n_acc & ~31;
     p.n_tile = cut.n_tile; p.full = cut.full; p.splits = cut.splits; p.items = cut.items;
@@ -980,8 +991,9 @@ int qw3::gemm_launch(qw3_w4_t w, const void* d_x, int64_t rows, void* d_y, qw3_w
     QW3_REQUIRE(rows >= 1 && rows <= (1 << 20), "qw3_gemm_w4a16: rows out of range");
     QW3_REQUIRE((reinterpret_cast<uintptr_t>(d_x) & 15) == 0, "qw3_gemm_w4a16: X must be 16-byte aligned");
     const W4Desc* d = w4_desc(w);
-    if (pair_wanted(d, rows, d_y, ws_struct(ws)))
-        return pair_launch(d, d_x, rows, d_y, ws_struct(ws), static_cast<cudaStream_t>(stream), epilogue);
+    PairCut pair = {};
+    if (pair_wanted(d, rows, d_y, ws_struct(ws), &pair))
+        return pair_launch(d, pair, d_x, rows, d_y, ws_struct(ws), static_cast<cudaStream_t>(stream), epilogue);
     GemmParams p = {};
     p.packed = d->packed;
     p.scale = d->scale; p.zp = d->zp; p.n_alloc = (int)d->n_alloc;
