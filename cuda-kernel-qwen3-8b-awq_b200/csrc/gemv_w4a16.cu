@@ -675,9 +675,14 @@ int gemv_launch(const W4Desc* d, const Qw3GemvArgs* a, const Workspace* ws, bool
     QW3_REQUIRE(smem <= 227 * 1024, "qw3_gemv_w4a16: in_dim=%d needs %zu bytes of shared memory", p.K, smem);
     int grid = ws->sm_count < WS_MAX_CTAS ? ws->sm_count : WS_MAX_CTAS;
     // A stage of 64 rows keeps all sixteen consumer warps of a CTA busy at once: a CTA with less than one is no faster and
-    // leaves one more set of partial sums to add (1536 x 512: 16 CTAs instead of 128).
+    // leaves one more set of partial sums to add; and whole stages never straddle two tiles of outputs.  One CTA a unit of 8 rows / one a
+    // stage, graph replays without dependent launch (us): 512 x 512 9.6 / 8.3 (8 CTAs), 1024 x 2048 12.3 / 9.0 (32), 1024 x 4096 12.6 /
+    // 10.4 (64), 4096 x 1536 11.1 / 10.2 (96), 2048 x 4096 11.5 / 10.7 (128), 3072 x 3072 15.2 / 10.7 (144).  Not where it saves too
+    // little: a column of 128 inputs (2048 x 128 9.4 / 10.2 us a call) and, within one tile, less than a sixteenth of the CTAs
+    // (1024 x 9088 17.05 / 17.23 with 142).
     const long long stages = (p.U + STAGE_UNITS - 1) / STAGE_UNITS;
-    if (grid > stages) grid = (int)stages;
+    const long long most = p.upt >= 32 && (p.n_tiles > 1 || stages <= grid - grid / 16) ? stages : p.U;
+    if (grid > most) grid = (int)most;
     if (uniform) {
         if (d->zp_integral) return launch_gemv<true, true>(d, p, grid, smem, pdl, st);
         return launch_gemv<true, false>(d, p, grid, smem, pdl, st);
