@@ -984,6 +984,10 @@ extern "C" int qw3_gemm_w4a16(qw3_w4_t w, const void* d_x, int64_t rows, void* d
     return qw3::gemm_launch(w, d_x, rows, d_y, ws, stream, QW3_EPI_STORE);
 }
 
+extern "C" int qw3_gemm_w4a16_epilogue(qw3_w4_t w, const void* d_x, int64_t rows, void* d_y, qw3_ws_t ws, int32_t epilogue, void* stream) {
+    return qw3::gemm_launch(w, d_x, rows, d_y, ws, stream, epilogue);
+}
+
 // The contraction with an optional epilogue (the engine's batched prompt phase fuses the residual add and the GeLU).
 int qw3::gemm_launch(qw3_w4_t w, const void* d_x, int64_t rows, void* d_y, qw3_ws_t ws, void* stream, int epilogue) {
     QW3_REQUIRE(w && d_x && d_y && ws, "qw3_gemm_w4a16: null argument");

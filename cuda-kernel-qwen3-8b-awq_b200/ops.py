@@ -86,6 +86,10 @@ def gemm_w4a16(w, ws, x, y):
     cabi.check(cabi.lib().qw3_gemm_w4a16(w.h, _ptr(x), x.shape[0], _ptr(y), ws.h, _stream()), "qw3_gemm_w4a16")
 
 
+def gemm_w4a16_epilogue(w, ws, x, y, epilogue):
+    cabi.check(cabi.lib().qw3_gemm_w4a16_epilogue(w.h, _ptr(x), x.shape[0], _ptr(y), ws.h, epilogue, _stream()), "qw3_gemm_w4a16_epilogue")
+
+
 def rmsnorm(x, gamma, eps=1e-6):
     out = torch.empty_like(x)
     cabi.check(cabi.lib().qw3_rmsnorm(_ptr(x), _ptr(gamma), x.numel(), eps, _ptr(out), _stream()), "qw3_rmsnorm")

@@ -138,6 +138,9 @@ int qw3_gemv_w4a16_noalloc_status(void* stream);
  * batched path; row r of Y equals qw3_gemv_w4a16 on row r of X within fp32 summation order.
  * X is [rows][in_dim], Y is [rows][out_dim]. */
 int qw3_gemm_w4a16(qw3_w4_t w, const void* d_x, int64_t rows, void* d_y, qw3_ws_t ws, void* stream);
+/* The same with the epilogues that the engine's prompt phase uses: QW3_EPI_STORE, QW3_EPI_RESIDUAL (Y = hadd(Y, product)) or
+ * QW3_EPI_GELU (of the product as fp16). */
+int qw3_gemm_w4a16_epilogue(qw3_w4_t w, const void* d_x, int64_t rows, void* d_y, qw3_ws_t ws, int32_t epilogue, void* stream);
 
 /* rmsNormKernel (Inference.cu:111-145), standalone. */
 int qw3_rmsnorm(const void* d_x, const void* d_gamma, int64_t n, float eps, void* d_out, void* stream);

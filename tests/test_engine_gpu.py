@@ -70,6 +70,27 @@ def test_small_model_batched_prefill(pkg, orc, cuda, small_dir):
     inf.close()
 
 
+@pytest.mark.parametrize("hidden,inter,heads,n_prompt", [(512, 1536, 4, 129), (1024, 2048, 8, 299), (2048, 1024, 16, 450)])
+def test_batched_prompts_through_the_pairs(pkg, orc, cuda, tmp_path, hidden, inter, heads, n_prompt):
+    """Prompts of more than 128 ids run on the contraction by CTA pairs: whole tiles, w2 split along K (second model) and wo and w1
+    (third).  Ids and logits as the token loop and the oracle give them."""
+    cfg_kw = dict(SMALL, hidden=hidden, inter=inter, heads=heads, layers=2, max_pos=512)
+    d = str(tmp_path)
+    orc.write_weight_dir(orc.default_config(**cfg_kw), SEED, d)
+    prompt = orc.gen_tokens(SEED, orc.TOKENS, n_prompt, SMALL["vocab"])
+    ids, logits, margins = _oracle_generate(orc, cfg_kw, SEED, d, prompt, 4)
+    inf = pkg.QWen3AWQInfer(d, keep_logits=1, **cfg_kw)
+    inf.set_batched_prefill(False)
+    loop_ids = inf.generateResponse(prompt, 4)
+    loop_logits = inf.last_logits()
+    inf.set_batched_prefill(True)
+    got = inf.generateResponse(prompt, 4)
+    assert got == [int(t) for t in ids] == loop_ids, f"margins {margins}"
+    assert _logits_close(inf.last_logits(), logits)
+    assert _logits_close(inf.last_logits(), loop_logits.astype(np.float16))
+    inf.close()
+
+
 @pytest.mark.parametrize("persistent", [2, 1, 0])
 def test_small_model_sample_first(pkg, orc, cuda, small_dir, persistent):
     prompt = orc.gen_tokens(SEED, orc.TOKENS, 6, SMALL["vocab"])

@@ -138,3 +138,30 @@ def test_gemm_pairs_sum_no_longer_than_one_cta(ops, orc, cuda, M, K, R):
     one = off[2:2 + R * M].view(R, M).cpu().numpy()
     pairs, ref = (got[rows] != want).sum(), (one[rows] != want).sum()
     assert ref > 100 and pairs <= 1.3 * ref
+
+
+@pytest.mark.parametrize("M,K,R", [(512, 512, 40), (512, 2048, 40),   # one CTA a tile, without and with its K split
+                                   (1024, 1024, 300),                 # pairs, whole tiles
+                                   (1024, 2048, 300), (384, 4096, 131),   # pairs, every tile split; an odd number of 128-output blocks
+                                   (19200, 4096, 130)])               # pairs, a whole wave and a split tile
+def test_gemm_epilogues(ops, orc, cuda, M, K, R):
+    """The residual add and the GeLU act on the product as fp16: they equal the same operation on what the plain call stores (which
+    the tests above hold to the oracle), the add bit by bit, the GeLU up to the last place of erf."""
+    p, s, z = orc.gen_linear(44, M, K)
+    X = orc.gen_normal_f16(44, orc.ACT, R * K).reshape(R, K)
+    got, w, ws = _gemm(ops, cuda, p, s, z, M, K, X)
+    rows = [0, R // 2, R - 1]
+    y32, y16 = orc.gemm_w4a16(p, s, z, M, K, X[rows])
+    _check(got[rows], y32, y16, f"{M}x{K} rows {R}", differ=0.05)
+    old = orc.gen_normal_f16(45, orc.ACT, R * M).reshape(R, M)
+    y = _to_dev(old, cuda)
+    ops.gemm_w4a16_epilogue(w, ws, _to_dev(X, cuda), y, ops.cabi.EPI_RESIDUAL)
+    assert np.array_equal(y.cpu().numpy().view(np.uint16), orc.add(old.ravel(), got.ravel()).reshape(R, M).view(np.uint16))
+    ops.gemm_w4a16_epilogue(w, ws, _to_dev(X, cuda), y, ops.cabi.EPI_GELU)
+    want = orc.gelu(got.ravel()).reshape(R, M)
+    d = _ulp_diff(y.cpu().numpy(), want)
+    # where 1 + erf cancels, a unit in the last place of erf (2^-24) times half the value is what is left of the result
+    near = np.abs(y.cpu().numpy().astype(np.float32) - want.astype(np.float32)) <= 2.0 ** -23 * np.abs(got.astype(np.float32))
+    assert ((d <= 1) | near).all()
+    ws.check()
+    assert ops.cabi.lib().qw3_gemm_w4a16_epilogue(w.h, y.data_ptr(), R, y.data_ptr(), ws.h, ops.cabi.EPI_ARGMAX, None) == ops.cabi.QW3_ERR_ARG
