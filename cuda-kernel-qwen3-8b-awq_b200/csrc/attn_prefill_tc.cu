@@ -17,7 +17,7 @@
 // Bound: the MMAs, 768 cycles per 128 x 64 scores (256 for S, 256 for each term of P), beside 512 cycles of exponentials.
 // All waits are bounded.  After one that gives up the error word is set, rows that are not finished are written as NaN, and the CTA
 // leaves when its copies and MMAs in flight are done.
-#include <mutex>
+#include <atomic>
 
 #include "tc05.cuh"
 
@@ -372,9 +372,12 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
     }
 }
 
-// qkv [rows][3 * hidden] (q rotated), caches [heads][max_pos][128], these three 16-byte aligned.
+// qkv [rows][3 * hidden] (q rotated), caches [heads][max_pos][128].
 int attn_prefill_tc_launch(const void* qkv, const void* kc, const void* vc, int heads, int hidden, long long max_pos, int pos0, int rows,
                            void* ctx, int* err, bool poll_once, cudaStream_t st) {
+    QW3_REQUIRE(((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(kc) | reinterpret_cast<uintptr_t>(vc)) & 15) == 0,
+                "qw3_attn_prefill: qkv and both caches must be 16-byte aligned from 16 rows on");
+    QW3_REQUIRE((reinterpret_cast<uintptr_t>(ctx) & 3) == 0, "qw3_attn_prefill: ctx must be 4-byte aligned from 16 rows on");
     CUtensorMap tm_q, tm_k, tm_v;
     const uint64_t qd[2] = {(uint64_t)hidden, (uint64_t)rows}, qs[1] = {(uint64_t)hidden * 6};
     const uint32_t qb[2] = {64, AT_ROWS};
@@ -385,15 +388,14 @@ int attn_prefill_tc_launch(const void* qkv, const void* kc, const void* vc, int 
     if (rc == QW3_OK) rc = encode_f16_map(&tm_k, kc, 3, kd, ks, kb);
     if (rc == QW3_OK) rc = encode_f16_map(&tm_v, vc, 3, kd, ks, kb);
     if (rc != QW3_OK) return rc;
-    static std::once_flag attr_once[64];
+    static std::atomic<bool> attr_set[64];   // per device: the kernel's shared-memory limit is raised once
     int dev = 0;
     QW3_CUDA(cudaGetDevice(&dev));
-    auto set_attr = [] {
-        cudaFuncSetAttribute(attn_prefill_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AT_SMEM);
-        cudaFuncSetAttribute(attn_prefill_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AT_SMEM);
-    };
-    if (dev >= 0 && dev < 64) std::call_once(attr_once[dev], set_attr);
-    else set_attr();
+    if (dev >= 64 || !attr_set[dev].load(std::memory_order_acquire)) {
+        QW3_CUDA(cudaFuncSetAttribute(attn_prefill_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AT_SMEM));
+        QW3_CUDA(cudaFuncSetAttribute(attn_prefill_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AT_SMEM));
+        if (dev < 64) attr_set[dev].store(true, std::memory_order_release);
+    }
     AttnParams p = {static_cast<const __half*>(qkv), static_cast<const __half*>(kc), static_cast<const __half*>(vc), max_pos,
                     static_cast<__half*>(ctx), hidden, pos0, rows, err};
     const dim3 grid(heads, (rows + 2 * AT_ROWS - 1) / (2 * AT_ROWS));

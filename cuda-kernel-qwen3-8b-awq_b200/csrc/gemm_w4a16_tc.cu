@@ -17,6 +17,7 @@
 // Within every group of 8 outputs the rows of A are stored in the order the lop3 unpack yields them
 // (0,4,1,5,2,6,3,7); the epilogue undoes that permutation when it computes the output index.
 // All mbarrier waits are bounded; a wait that gives up sets the workspace error word.
+#include <atomic>
 #include <cstdlib>
 #include <mutex>
 
@@ -944,17 +945,16 @@ static int pair_launch(const W4Desc* d, const PairCut& cut, const void* d_x, lon
     CUtensorMap tmap_x;
     const int rc = encode_rows(&tmap_x, d_x, rows, d->K, p.n_tile / 2);
     if (rc != QW3_OK) return rc;
-    static std::once_flag attr_once[16];
+    static std::atomic<bool> attr_set[64];   // per device: the kernels' shared-memory limit is raised once
     int dev = 0;
     QW3_CUDA(cudaGetDevice(&dev));
-    auto set_attr = [] {
-        cudaFuncSetAttribute(gemm_w4a16_pair_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GP_SMEM);
-        cudaFuncSetAttribute(gemm_w4a16_pair_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GP_SMEM);
-        cudaFuncSetAttribute(gemm_w4a16_pair_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GP_SMEM);
-        cudaFuncSetAttribute(gemm_w4a16_pair_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GP_SMEM);
-    };
-    if (dev < 16) std::call_once(attr_once[dev], set_attr);
-    else set_attr();
+    if (dev >= 64 || !attr_set[dev].load(std::memory_order_acquire)) {
+        QW3_CUDA(cudaFuncSetAttribute(gemm_w4a16_pair_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GP_SMEM));
+        QW3_CUDA(cudaFuncSetAttribute(gemm_w4a16_pair_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GP_SMEM));
+        QW3_CUDA(cudaFuncSetAttribute(gemm_w4a16_pair_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GP_SMEM));
+        QW3_CUDA(cudaFuncSetAttribute(gemm_w4a16_pair_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GP_SMEM));
+        if (dev < 64) attr_set[dev].store(true, std::memory_order_release);
+    }
     const unsigned grid = 2u * (unsigned)(p.items < pairs ? p.items : pairs);
     if (d->zp_integral) {
         if (d->uniform) gemm_w4a16_pair_kernel<true, true><<<grid, GP_THREADS, GP_SMEM, st>>>(tmap_x, p);

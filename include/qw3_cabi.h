@@ -160,8 +160,8 @@ int qw3_attn_decode(const void* d_q, const void* d_k_cache, const void* d_v_cach
 /* The same attention for a block of `rows` consecutive prompt positions pos0 .. pos0 + rows - 1 (the batched prompt phase;
  * the reference runs attentionKernel once per prompt token, Inference.cu:1304-1343): row r of d_qkv ([rows][3 * heads * 128]
  * fp16, q in the first third, after RoPE) attends cache rows 0 .. pos0 + r, which must already hold the block's own k / v
- * rows; d_ctx is [rows][heads * 128] fp16.  From 16 rows on a tiled tensor-core kernel runs (64 query rows share each tile
- * of 64 cache rows), below that one CTA per row. */
+ * rows; d_ctx is [rows][heads * 128] fp16.  From 16 rows on a tensor-core kernel runs (256 query rows share each tile of 64
+ * cache rows), which needs d_qkv and the caches on 16 bytes and d_ctx on 4 (else QW3_ERR_ARG); below that one CTA per row. */
 int qw3_attn_prefill(const void* d_qkv, const void* d_k_cache, const void* d_v_cache, int32_t heads, int32_t head_dim,
                      int64_t max_pos, int32_t pos0, int32_t rows, void* d_ctx, void* stream);
 /* Companion of qw3_attn_prefill, which takes no workspace (as qw3_gemv_w4a16_noalloc_status is of the GEMV without one): a wait that

@@ -69,6 +69,14 @@ def test_null_arguments_are_rejected_without_a_gpu(pkg):
     assert L.qw3_destroy(None) == cabi.QW3_OK
 
 
+def test_prompt_attention_names_a_misaligned_pointer_without_a_gpu(pkg):
+    cabi = pkg.cabi
+    L = cabi.lib()
+    for qkv, k, v, ctx, what in ((8, 256, 256, 256, b"16-byte"), (256, 264, 256, 256, b"16-byte"), (256, 256, 258, 256, b"16-byte"), (256, 256, 256, 258, b"4-byte")):
+        assert L.qw3_attn_prefill(qkv, k, v, 1, 128, 64, 0, 16, ctx, None) == cabi.QW3_ERR_ARG
+        assert what in L.qw3_last_error()
+
+
 def test_product_code_does_not_reach_the_oracle():
     """Nothing in the package or the headers may import, link or name the oracle."""
     pkg_dir = os.path.join(ROOT, "cuda-kernel-qwen3-8b-awq_b200")
