@@ -8,12 +8,13 @@
 //               lies in the cache
 //   warps 4..7, 8..11   one row a thread of the upper / lower tile: S from tensor memory, online softmax, P back in its place
 // Tensor memory, per tile: O 128 columns, two S buffers of 64.  P goes in as TWO fp16 terms (P = hi + lo, lo the rounding error of
-// hi): 32 + 32 columns, exactly the room of the S it comes from, so the probabilities keep 22 bits as 32-bit arithmetic does.
+// hi): 32 + 32 columns, exactly the room of the S it comes from.  That is 22 bits from 2^-3 on, below it an absolute error of 2^-25 (the
+// last place of fp16), where a row's largest P lies between 1 and 256.
 // While the threads work on one S the tensor cores compute the other and the other tile's products.  O is rescaled (a pass of
 // tensor memory -> registers -> tensor memory) only when a row's maximum has grown by more than 8 powers of two since the
 // last time: P then stays at or below 256 and the quotient O / l is the same.
-// 1953 rows at position 2048, 32 heads: 590 us with warp-level MMAs (mma.sync, 64 rows a CTA), 160 now, 0.36 of the measured bf16
-// rate in useful operations (the second term of P and the masked halves of the diagonal tiles are not counted).
+// 1953 rows at position 2048, 32 heads, a call among others: 590 us with warp-level MMAs (mma.sync, 64 rows a CTA), 163 now, 0.36 of the
+// measured bf16 rate in useful operations (the second term of P and the masked halves of the diagonal tiles are not counted).
 // Bound: the MMAs, 768 cycles per 128 x 64 scores (256 for S, 256 for each term of P), beside 512 cycles of exponentials.
 // All waits are bounded.  After one that gives up the error word is set, rows that are not finished are written as NaN, and the CTA
 // leaves when its copies and MMAs in flight are done.

@@ -330,9 +330,9 @@ __global__ void gemm_splitk_reduce_kernel(const float* __restrict__ part, int sp
 }
 
 // ---- CTA pairs ------------------------------------------------------------------------------------------------------------------
-// More than 128 rows, or more output tiles than pairs (pair_wanted).  2048 rows of 12288 x 4096: 246 us before, 189 now (0.65 of the
-// measured bf16 rate); 64 rows of 151936 x 4096: 264 before, 205 now.  Bound: a K block takes 0.35 us from the unpack warps to the
-// freed stage whatever the row count (0.25 us with the unpacking left out), above the 0.28 us its MMAs take at 256 rows.
+// Most calls of more than 128 rows, and those with more output tiles than pairs (pair_wanted).  Back to back, one-CTA kernel / pairs:
+// 2048 rows of 12288 x 4096 202 / 158 us (0.76 of the measured bf16 rate), 64 rows of 151936 x 4096 250 / 193.  Bound: a K block takes
+// 0.33 us from the unpack warps to the freed stage whatever the row count, 0.39 at 256 rows, where its MMAs take 0.28.
 // Two SMs of a cluster work on one tile of 256 outputs x n_tile rows (tcgen05 cta_group::2): each CTA unpacks operand A for its
 // own 128 outputs and holds half of the activation rows, so that a K block moves half the operand-B bytes through an SM's
 // shared memory (A 16 KB written + 16 KB read, B 16 KB + 16 KB, in the 512 cycles the MMAs take at 256 rows) and half through L2.
