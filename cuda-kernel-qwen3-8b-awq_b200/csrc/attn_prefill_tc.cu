@@ -152,11 +152,11 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
             for (int t = 0; t < 2; ++t)
                 for (int h = 0; h < 2; ++h)
                     tma_load_2d(smem_u32(q_s + t * AT_Q_BYTES + h * (AT_Q_BYTES / 2)), &tm_q, head * 128 + 64 * h, r0 + AT_ROWS * t, q_full);
-            int issued[2] = {0, 0};   // tiles of K and V
-            for (int j = 0; j < n_tiles && ok; ++j) {
+            int j = 0, kv = 0;
+            for (; j < n_tiles; ++j) {
                 const int s = j % AT_STAGES;
                 const uint32_t lap = (uint32_t)(j / AT_STAGES);
-                for (int kv = 0; kv < 2 && ok; ++kv) {
+                for (kv = 0; kv < 2; ++kv) {
                     const uint32_t full = (kv ? v_full : k_full) + 8 * s, empty = (kv ? v_empty : k_empty) + 8 * s;
                     uint8_t* dst = (kv ? v_s : k_s) + s * AT_KV_BYTES;
                     if (lap > 0) ok = wait(empty, (lap - 1) & 1u);
@@ -165,20 +165,22 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
                     mbar_expect_tx(full, AT_KV_BYTES);
                     for (int h = 0; h < 2; ++h)
                         tma_load_3d(smem_u32(dst + h * (AT_KV_BYTES / 2)), kv ? &tm_v : &tm_k, 64 * h, j * AT_KEYS, head, full);
-                    ++issued[kv];
                 }
+                if (!ok) break;
             }
             // drain: the last release arrivals land before the CTA may leave
-            for (int j = n_tiles < AT_STAGES ? 0 : n_tiles - AT_STAGES; j < n_tiles && ok; ++j) {
-                const uint32_t parity = (uint32_t)(j / AT_STAGES) & 1u;
-                ok = wait(k_empty + 8 * (j % AT_STAGES), parity) && wait(v_empty + 8 * (j % AT_STAGES), parity);
+            for (int i = n_tiles < AT_STAGES ? 0 : n_tiles - AT_STAGES; i < n_tiles && ok; ++i) {
+                const uint32_t parity = (uint32_t)(i / AT_STAGES) & 1u;
+                ok = wait(k_empty + 8 * (i % AT_STAGES), parity) && wait(v_empty + 8 * (i % AT_STAGES), parity);
             }
             if (!ok) {
                 give_up(0x30021);
                 mbar_wait(q_full, 0);   // the copies in flight
-                for (int kv = 0; kv < 2; ++kv)
-                    for (int j = max(issued[kv] - AT_STAGES, 0); j < issued[kv]; ++j)
-                        mbar_wait((kv ? v_full : k_full) + 8 * (j % AT_STAGES), (uint32_t)(j / AT_STAGES) & 1u);
+                for (int t = 0; t < 2; ++t) {
+                    const int asked = j < n_tiles && t < kv ? j + 1 : j;   // tiles of K, of V
+                    for (int i = max(asked - AT_STAGES, 0); i < asked; ++i)
+                        mbar_wait((t ? v_full : k_full) + 8 * (i % AT_STAGES), (uint32_t)(i / AT_STAGES) & 1u);
+                }
             }
         }
         __syncwarp();
@@ -233,8 +235,10 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
                 }
             }
             if (!ok) give_up(0x30022);
-            umma_commit(drain);   // whoever gives up: the CTA does not leave before its MMAs are done
-            mbar_wait(drain, 0);
+            if (POLL_ONCE || !ok || *s_dead != 0) {   // the MMAs in flight (a wait that gives up later does so long after they are done)
+                umma_commit(drain);
+                mbar_wait(drain, 0);
+            }
         }
         __syncwarp();
     } else if (warp >= 4) {
@@ -245,8 +249,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
         const int pos_first = pos - lane;                                      // of the warp's first row
         const float c = (float)(1.4426950408889634 / 11.313708498984761);      // log2(e) / sqrt(128), Inference.cu:218
         float m = -INFINITY, mc = 0.0f, l = 0.0f;   // m: maximum in use (raw scores), mc = m c
-        float mr = 0.0f;                            // m c - mc where that is not small
-        bool coarse = false, ok = true;             // some row of the warp has mr
+        float mr = 0.0f, off = 0.0f;                // m c - mc where that is not small, and then off = 0 and m is taken off s; else off = mc
+        bool ok = true;
         for (int j = 0; j < n_tiles && ok; ++j) {
             const int b = j & 1;
             ok = __all_sync(0xffffffffu, *s_dead == 0 && wait(s_full + 16 * t + 8 * b, (uint32_t)(j >> 1) & 1u));
@@ -268,7 +272,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
 #pragma unroll
             for (int e = 4; e < 64; ++e) mx[e & 3] = fmaxf(mx[e & 3], s[e]);
             const float mt = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
-            if (__any_sync(0xffffffffu, (mt - m) * c > 8.0f)) {   // rare after the first tile
+            if (__any_sync(0xffffffffu, (mt - m) * c > 8.0f || mr != 0.0f)) {   // rare after the first tile
                 const float mn = fmaxf(m, mt), nmc = mn == -INFINITY ? 0.0f : mn * c;
                 const float nmr = fabsf(nmc) >= 1048576.0f ? fmaf(mn, c, -nmc) : 0.0f;
                 const float f = m == -INFINITY ? 0.0f : ex2((mc - nmc) + (mr - nmr));
@@ -290,14 +294,12 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
                 m = mn;
                 mc = nmc;
                 mr = nmr;
-                coarse = __any_sync(0xffffffffu, mr != 0.0f);
-            }
-            float sc = c, off = mc;
-            if (coarse) {
+                off = mr != 0.0f ? 0.0f : mc;
+                if (__any_sync(0xffffffffu, mr != 0.0f)) {
+                    const float base = mr != 0.0f ? m : 0.0f;
 #pragma unroll
-                for (int e = 0; e < 64; ++e) s[e] = fmaf(s[e], c, -mc) - mr;
-                sc = 1.0f;
-                off = 0.0f;
+                    for (int e = 0; e < 64; ++e) s[e] -= base;
+                }
             }
             float ls[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
@@ -305,7 +307,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
                 uint32_t hi[16], lo[16];
 #pragma unroll
                 for (int e = 0; e < 16; ++e) {
-                    const float a0 = ex2(fmaf(s[32 * h + 2 * e], sc, -off)), a1 = ex2(fmaf(s[32 * h + 2 * e + 1], sc, -off));
+                    const float a0 = ex2(fmaf(s[32 * h + 2 * e], c, -off)), a1 = ex2(fmaf(s[32 * h + 2 * e + 1], c, -off));
                     ls[(2 * e) & 3] += a0;
                     ls[(2 * e + 1) & 3] += a1;
                     const __half2 hh = __floats2half2_rn(a0, a1);
