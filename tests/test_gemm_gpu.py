@@ -165,3 +165,15 @@ def test_gemm_epilogues(ops, orc, cuda, M, K, R):
     assert ((d <= 1) | near).all()
     ws.check()
     assert ops.cabi.lib().qw3_gemm_w4a16_epilogue(w.h, y.data_ptr(), R, y.data_ptr(), ws.h, ops.cabi.EPI_ARGMAX, None) == ops.cabi.QW3_ERR_ARG
+
+
+@pytest.mark.parametrize("M,K,R,integral", [
+    (128, 1024, 129, True),     # row tiles of 32, four accumulators; one row in the last tile; half of the pair without outputs
+    (640, 1024, 900, False),    # 64, four
+    (896, 4096, 257, True),     # 96, three, K in six parts
+    (384, 4096, 641, False),    # 128, three
+    (896, 4096, 300, True),     # 160, three, K in seven parts
+    (384, 4096, 513, True), (1152, 2048, 385, False), (3712, 512, 901, True)])   # 192, 224 and 256, two
+def test_gemm_pairs_widths(ops, orc, cuda, M, K, R, integral):
+    """The cuts that the times choose: every width of a row tile and number of accumulators, with rows that do not fill the last tile."""
+    test_gemm_pairs_edges(ops, orc, cuda, M, K, R, integral)
