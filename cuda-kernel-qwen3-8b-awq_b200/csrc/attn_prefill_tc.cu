@@ -13,7 +13,7 @@
 // While the threads work on one S the tensor cores compute the other and the other tile's products.  O is rescaled (a pass of
 // tensor memory -> registers -> tensor memory) only when a row's maximum has grown by more than 8 powers of two since the
 // last time: P then stays at or below 256 and the quotient O / l is the same.
-// 1953 rows at position 2048, 32 heads, a call among others: 590 us with warp-level MMAs (mma.sync, 64 rows a CTA), 163 now, 0.36 of the
+// 1953 rows at position 2048, 32 heads, a call among others: 590 us with warp-level MMAs (mma.sync, 64 rows a CTA), 164 now, 0.36 of the
 // measured bf16 rate in useful operations (the second term of P and the masked halves of the diagonal tiles are not counted).
 // Bound: the MMAs, 768 cycles per 128 x 64 scores (256 for S, 256 for each term of P), beside 512 cycles of exponentials.
 // All waits are bounded.  After one that gives up the error word is set, rows that are not finished are written as NaN, and the CTA
